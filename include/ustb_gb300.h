@@ -170,7 +170,7 @@ enum {
     USTB_WIN_TUKEY25 = 4, USTB_WIN_TUKEY50 = 5, USTB_WIN_TUKEY75 = 6, USTB_WIN_TRIANGLE = 9
 };
 
-/* Pixels per tile of the fast path (one CTA). */
+/* Pixels per tile of the fast path (two CTAs). */
 #define USTB_TILE_PIXELS 512
 
 /*
@@ -281,7 +281,7 @@ typedef struct {
 
 /*
  * Batched, persistent form of ustb_das_fast: every request is cut into
- * (frame, tile) work items and one CTA per SM pulls items from a queue until all
+ * (frame, tile) work items and two CTAs per SM pull items from a queue until all
  * are done, so requests of different scans, probes, frame counts and sizes share
  * one launch and balance across the GPU (one launch per kernel variant, i.e. per
  * dimension / real-complex / epilogue combination present).  Each request's
@@ -314,9 +314,9 @@ int ustb_das_fast_batch_ws(const ustb_das_request* reqs, int32_t n, uint64_t* sc
 
 /*
  * ustb_das_fast_batch / _ws with a bound on the persistent launch's CTAs:
- * max_ctas > 0 runs at most that many CTAs (one per SM), leaving the other SMs to
- * launches on other streams, e.g. small requests served while a large one runs;
- * 0 = one CTA per SM.  workspace may be NULL (library pool, as
+ * max_ctas > 0 takes at most the room of that many whole SMs (two half-SM CTAs each),
+ * leaving the rest to launches on other streams, e.g. small requests served while a
+ * large one runs; 0 = every SM.  workspace may be NULL (library pool, as
  * ustb_das_fast_batch).  No reference counterpart (the reference serves nothing).
  */
 int ustb_das_fast_batch_ex(const ustb_das_request* reqs, int32_t n, uint64_t* scratch, void* workspace,

@@ -15,9 +15,8 @@ stage shape sets how often the receive geometry (per pixel and channel) and the
 transmit geometry (per pixel and wave) are formed, and how many of a stage's slots
 a short wave sequence fills (11 waves fill 11 of 16 slots of a waves-outer chunk,
 11 of 12 of channels-outer chunks).  Fixed by the kernel, because measurement showed
-no gain from changing them: the samples per slot (160; 104- and 80-entry slots with
-3- and 4-deep buffer rings ran at the same speed) and one 512-thread CTA per SM (the
-register file's limit); the persistent launches use one CTA per SM unless a caller
+no gain from changing them: two buffers of 32 slots per stage and two 256-thread CTAs
+per SM (the register file's limit); the persistent launches use every SM unless a caller
 bounds them to share the GPU with other streams (``fast.das_fast_batch(max_ctas=)``).
 
 Each candidate is timed with CUDA events on the caller's data; the fastest is

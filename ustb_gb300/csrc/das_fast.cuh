@@ -1,0 +1,52 @@
+// What the host side of the fast path (das_fast.cu) shares with its kernels
+// (das_fast_kernel.cuh, instantiated by das_fast_*.cu so that they compile in parallel).
+#pragma once
+
+#include "common.cuh"
+
+namespace ustb {
+
+constexpr int kTile = USTB_TILE_PIXELS;
+
+struct Params {
+    const void* entries;  // [F][W][N][Lp] interpolation entries (float4 complex, float2 real)
+    int64_t L, Lp, N, W, F, P;
+    const float* el;
+    const float* px;
+    const int32_t* tiles;
+    int64_t n_tiles;
+    const ustb_wave* waves;
+    const float* tx_delay_tab;
+    const float* tx_apo_tab;
+    const float* rx_apo_tab;
+    const float2* pix_phase;
+    float fs, t0, fd, inv_c, lens;
+    double fd_fs;  // fd / fs
+    int64_t wave_step, frame_step;  // entries from a wave (a frame) to the next
+    int rx_window;
+    float win_r1, win_a, win_e, win_b, win_c, win_d;  // see window_coeffs()
+    float fnx, fny, minx, miny, maxx, maxy;
+    int rx_origin;
+    float ox, oy, oz;
+    float cf_thr;
+    void* cube;
+    float2* o_das;
+    float* o_cf;
+    float2* o_cfimg;
+    float* o_sdmas;
+    int64_t rx_f, w_f, f_f;
+    uint32_t* flags;
+    int split;  // grid kernel, dimension.both: CTAs per tile (parts of the stage list, 1-4); 0 = auto
+    int shape;  // stage shape (Shape<> index)
+    int fpi;    // persistent kernel: frames per work item (one tile, consecutive frames)
+};
+
+// Kernel variant of (dimension, epilogue, stage shape) for one request kind: one grid
+// launch of reqs[0] (BATCH false) or one persistent launch of n requests.
+template <bool CPLX, bool BATCH>
+int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t* frames, int n,
+                 unsigned long long* counter, int64_t nt, int64_t F, cudaStream_t s, int max_ctas);
+
+constexpr int kMaxBatch = 40;  // requests per persistent launch
+
+}  // namespace ustb

@@ -82,7 +82,7 @@ struct ustb_server_s {
     bool sched_exited = false;   // the scheduler has launched everything it will
     int64_t budget = 0;
     int64_t large_units = 0;  // requests above this many units go to the large stream
-    int large_ctas = 0;       // persistent CTAs of a large launch (0: one per SM)
+    int large_ctas = 0;       // SMs' worth of persistent CTAs of a large launch (0: every SM)
     int large_flight = 0;     // large launches not yet completed
     int max_batch = 1;
     int device = 0;
@@ -116,7 +116,7 @@ bool ustb_server_s::is_large(const Job& j) const {
     return r.L > 0 && (double)r.geometry->n_pixels * r.N * r.W * r.F > (double)large_units;
 }
 
-// Launch a batch on stream i (max_ctas 0: one persistent CTA per SM).
+// Launch a batch on stream i (max_ctas 0: every SM).
 int ustb_server_s::launch(const std::vector<Job>& jobs, int i, int max_ctas, Batch& b) {
     std::vector<ustb_das_request> reqs(jobs.size());
     for (size_t k = 0; k < jobs.size(); ++k) ustb::plan_request(jobs[k].plan, jobs[k].ch, &jobs[k].out, &reqs[k]);

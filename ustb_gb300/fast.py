@@ -530,8 +530,8 @@ def das_fast_batch(requests: Sequence[Request], scratch: Optional[torch.Tensor] 
     ``workspace``: optional uint8 device tensor of at least ``workspace_bytes(requests)``
     bytes (256-byte aligned, as torch allocations are) that holds the interpolation
     entries; without it the library allocates them from its own pool.
-    ``max_ctas``: at most this many persistent CTAs (0 = one per SM), so that launches
-    on other streams can use the remaining SMs meanwhile."""
+    ``max_ctas``: room of at most this many whole SMs for the persistent CTAs, two per SM
+    (0 = every SM), so that launches on other streams can use the rest meanwhile."""
     if not requests:
         return scratch
     dev = requests[0].ch.device
