@@ -60,3 +60,49 @@ def test_demodulation_of_rf_at_any_address(cuda_dev, dtype, shift):
     got = preprocess.demodulate(flat[shift:].view(6, 403), 20e6, 0.0, 5e6, taps, 2)
     want = O.fast_demodulation_f64(rf.T.astype(np.float64), 20e6, 0.0, 5e6, taps, 2)
     assert rel(iq(got), want.T) <= 1e-5
+
+
+def cube_of(rng, P, K, F=1):
+    c = rng.standard_normal((F, K, P)) + 1j * rng.standard_normal((F, K, P)) + 1.5 * rng.standard_normal((F, 1, P))
+    c[:, :, 0] = 0  # a silent pixel
+    return c.astype(np.complex64)
+
+
+@pytest.mark.parametrize("K", [2, 3, 7, 64, 130, 1024])
+@pytest.mark.parametrize("P, F", [(65, 2), (300, 1)])
+def test_phase_coherence_counts(cuda_dev, K, P, F):
+    rng = np.random.default_rng(K + P)
+    c = cube_of(rng, P, K, F)
+    w = rng.uniform(0, 1, (K, P)).astype(np.float32)
+    w[rng.random((K, P)) < 0.3] = 0
+    w[0] = 0.5  # every pixel keeps a weight
+    got = postprocess.phase_coherence_factor(torch.from_numpy(c[:, None]).to(cuda_dev), torch.from_numpy(w).to(cuda_dev))
+    for f in range(F):
+        fca, fcc, img = O.phase_coherence_factor_f64(c[f].T, w.T)
+        assert np.max(np.abs(got["FCA"][f].cpu().numpy() - fca)) <= 1e-4
+        assert np.max(np.abs(got["FCC"][f].cpu().numpy() - fcc)) <= 1e-4
+        assert rel(got["image"][f].cpu().numpy(), img) <= 1e-4
+
+
+def test_phase_coherence_of_agreeing_and_extreme_values(cuda_dev):
+    """Phases that agree closely (at any angle), and magnitudes whose squares leave FP32."""
+    rng = np.random.default_rng(1)
+    K, P = 48, 130
+    ang = np.linspace(-np.pi, np.pi, P)[None, :] + 1e-3 * rng.standard_normal((K, P))
+    mag = 10.0 ** rng.uniform(-25, 25, (1, P))
+    c = (mag * np.exp(1j * ang)).astype(np.complex64)
+    got = postprocess.phase_coherence_factor(torch.from_numpy(c[None, None]).to(cuda_dev))
+    fca, fcc, _ = O.phase_coherence_factor_f64(c.T)
+    assert np.max(np.abs(got["FCA"][0].cpu().numpy() - fca)) <= 1e-4
+    assert np.max(np.abs(got["FCC"][0].cpu().numpy() - fcc)) <= 1e-4
+
+
+@pytest.mark.parametrize("M0, K", [(0, 2), (1, 5), (2, 3), (3, 4), (4, 5), (4, 64), (5, 11), (6, 7), (7, 8), (7, 1024)])
+def test_generalized_coherence_counts(cuda_dev, M0, K):
+    rng = np.random.default_rng(M0 * 100 + K)
+    c = cube_of(rng, 131, K, 2)
+    got = postprocess.generalized_coherence_factor(torch.from_numpy(c[:, None]).to(cuda_dev), M0)
+    for f in range(2):
+        g, img = O.generalized_coherence_factor_f64(c[f].T, M0)
+        assert np.max(np.abs(got["GCF"][f].cpu().numpy() - g)) <= 1e-5
+        assert rel(got["image"][f].cpu().numpy(), img) <= 1e-5
