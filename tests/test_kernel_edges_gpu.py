@@ -106,3 +106,22 @@ def test_generalized_coherence_counts(cuda_dev, M0, K):
         g, img = O.generalized_coherence_factor_f64(c[f].T, M0)
         assert np.max(np.abs(got["GCF"][f].cpu().numpy() - g)) <= 1e-5
         assert rel(got["image"][f].cpu().numpy(), img) <= 1e-5
+
+
+@pytest.mark.parametrize("M, L, K", [(2, 1, 0), (9, 4, 2), (40, 32, 1), (64, 32, 5), (73, 20, 0), (130, 32, 9), (256, 32, 1)])
+@pytest.mark.parametrize("fb", [False, True])
+def test_capon_channel_counts(cuda_dev, M, L, K, fb):
+    rng = np.random.default_rng(M + K)
+    nz, nx = 9, 2
+    d = 0.3 * (rng.standard_normal((nz, nx, M)) + 1j * rng.standard_normal((nz, nx, M)))
+    d += np.exp(1j * 0.3 * np.arange(M)) * rng.standard_normal((nz, nx, 1))
+    ap = np.ones((nz, nx, M))
+    for iz in range(nz):  # apertures that start and end anywhere in the tiles
+        ap[iz, :, :min(iz, M - 2)] = 0
+        ap[iz, 1, M - min(2 * iz, (M - 2) // 2):] = 0
+    cube = torch.from_numpy(np.ascontiguousarray(d.transpose(2, 1, 0).reshape(1, 1, M, nz * nx)).astype(np.complex64))
+    apod = torch.from_numpy(np.ascontiguousarray(ap.transpose(2, 1, 0).reshape(M, nz * nx)).astype(np.float32))
+    out = postprocess.capon_minimum_variance(cube.to(cuda_dev), apod.to(cuda_dev), nz, nx, L, K, 1e-2,
+                                             doForwardBackward=fb)
+    want = O.capon_f64(d, ap, L, K, 1e-2, fb=fb)
+    assert rel(out[0].cpu().numpy().reshape(nx, nz).T, want) <= 1e-3

@@ -1,5 +1,5 @@
 // Capon minimum-variance beamforming on a kept channel cube
-// (+postprocess/capon_minimum_variance.m:117-177), one warp per pixel.
+// (+postprocess/capon_minimum_variance.m:117-177), one warp per group of pixels.
 //
 // For pixel (iz, ix) of a scan grid with depth fastest, over the M values x[c] of
 // its channels (or waves) and the rows r of its depth window [iz-K, iz+K] (clipped):
@@ -11,11 +11,23 @@
 //   w = (R + I regCoef/L trace R)^-1 1 / (1^T (...)^-1 1),
 //   z = Ma / (Ma - L + 1) * sum_l conj(w)^T conj(x_iz[l:l+L])   (w' * x', as written).
 //
-// R is accumulated in shared memory along its diagonals: lane d owns diagonal d and
-// walks it with a sliding window, G(i+1, i+1+d) = G(i, i+d) + conj(x[l1+i+1]) x[l1+i+1+d]
-// - conj(x[l0+i]) x[l0+i+d], so a row costs (#l + 2L) products per lane instead of
-// #l * L.  The system is solved by a Cholesky factorisation R = U^H U in shared
-// memory, lanes over columns.
+// Summed over the rows first, R needs only the band P(c, d) = sum_r conj(X_r[c]) X_r[c + d],
+// d < L, of the channels' Gram matrix:
+//   R[i][i + d] = sum_{l = a}^{b - L + 1} P(l + i, d).
+// The band is cut into 8 x 8 tiles (30 for 64 channels), one per lane with its sums in
+// registers, so a row costs 16 shared-memory values per 64 products.  One warp takes up to
+// 4 neighbouring pixels of a depth column: the rows their windows share are summed once and
+// stay in registers, each pixel adds its own few rows.  Each lane then walks one diagonal
+// of P with a compensated sliding sum.  The system is solved by a Cholesky factorisation
+// R = U^H U, one column per lane and four rows at a time, the forward substitution carried
+// along, and a backward substitution with one unknown per lane.
+//
+// Latency-bound: 8 warps per SM (the tiles take 255 registers), 41 % issue.  GB300, 131072
+// pixels of 64 channels, 32-element subarrays, 15 rows: 2.51 ms; 5.57 ms with each row's
+// diagonals slid through shared memory and the triangular solves on one lane.  Not kept:
+// the factorisation unrolled with the column in registers (3.9 ms together with pixel
+// groups: the warps wait for instructions), packed pairs for the tiles (2.83 ms against
+// 2.69 ms), 12 warps of 168 registers (2.80 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,9 +37,25 @@
 
 namespace {
 
-constexpr int kLMax = 32;        // subarray length <= one lane per diagonal
-constexpr int kWarps = 4;        // pixels per CTA
+constexpr int kLMax = 32;        // subarray length <= one lane per diagonal and column
+constexpr int kWarps = 4;        // pixels per CTA at most
 constexpr int kMMax = 256;       // channels per pixel
+constexpr int kTileC = 8;        // channels per tile side
+constexpr int kTileStride = 20;  // words per staged block of 8 channels: 8 real, 8 imaginary parts, padding (the
+                                 // tiles' 16-byte loads hit distinct banks)
+constexpr int kRows = 8;         // rows staged at a time
+constexpr int kGroup = 4;        // pixels per warp at most
+constexpr int kBand = kLMax + 2;  // stride of the band and of R in shared memory
+
+// Words of shared memory per warp: staged rows, the band P (its space then takes R and U)
+// and the pixel's own row.
+__host__ __device__ __forceinline__ int blocks_of(int M) { return (M + kTileC - 1) / kTileC; }
+__host__ __device__ __forceinline__ int band_offset(int M) { return kRows * blocks_of(M) * kTileStride; }
+__host__ __device__ __forceinline__ int own_offset(int M) {
+    const int band = 2 * blocks_of(M) * kTileC * kBand, R = 2 * kLMax * kBand;
+    return band_offset(M) + (band > R ? band : R);
+}
+__host__ __device__ __forceinline__ int warp_words(int M) { return (own_offset(M) + 2 * M + 3) & ~3; }
 
 struct CaponArgs {
     int64_t nz, nx, F, M;
@@ -36,211 +64,349 @@ struct CaponArgs {
     float crit;            // active-element criterion
     float reg;             // regularisation coefficient
     int fb;                // forward-backward averaging
+    int group;             // neighbouring pixels (in depth) per warp, 1 .. kGroup
 };
 
 __device__ __forceinline__ float2 cmul_conj(float2 a, float2 b) {  // conj(a) * b
     return make_float2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
 
-__global__ void __launch_bounds__(32 * kWarps) capon_kernel(const float2* __restrict__ cube,
-                                                            const float* __restrict__ apod, float2* __restrict__ out,
-                                                            const CaponArgs a) {
-    __shared__ float2 sR[kWarps][kLMax][kLMax + 1];
-    __shared__ float2 srow[kWarps][kMMax];
-    __shared__ float2 sv[kWarps][kLMax];
-    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float2 (*R)[kLMax + 1] = sR[wi];
-    float2* row = srow[wi];
-    float2* v = sv[wi];
-    const int64_t P = a.nz * a.nx;
-    const int64_t total = P * a.F;
-    const int M = (int)a.M;
-    for (int64_t t = (int64_t)blockIdx.x * kWarps + wi; t < total; t += (int64_t)gridDim.x * kWarps) {
-        const int64_t f = t / P, p = t - f * P;
-        const int64_t ix = p / a.nz, iz = p - ix * a.nz;
-        const float2* base = cube + f * a.M * P;  // [M][P]
-        // active channels, all-zero test and the plain sum of the pixel's own row
-        int first = M, last = -1, cnt = 0;
-        bool any = false;
-        float2 sum = make_float2(0.f, 0.f);
-        for (int c = lane; c < M; c += 32) {
-            const float2 x = __ldg(base + (int64_t)c * P + p);
-            any |= hypotf(x.x, x.y) > 2.220446049250313e-16f;
-            sum.x += x.x;
-            sum.y += x.y;
-            if (fabsf(__ldg(apod + (int64_t)c * P + p)) > a.crit) {
-                first = min(first, c);
-                last = max(last, c);
-                ++cnt;
+__device__ __forceinline__ float2 shfl2(float2 v, int src) {
+    return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// The Capon value of one pixel from its band P (rows from channel c0 on): R, its
+// factorisation, the weights and their sum over the pixel's own row.  `start`: l0 - c0.
+__device__ __forceinline__ float2 capon_value(float2* band, const float2* own, const CaponArgs& a, int lane, int L,
+                                              int cnt, int start, int l0, int l1) {
+    // ---- R along its diagonals: lane d slides over diagonal d ----
+    const float norm = 1.f / ((float)(2 * a.K + 1) * (float)(cnt - L + 1));
+    {
+        const float2* Pd = band + start * kBand + lane;  // P(l0 + i, d) at i * kBand
+        const int nl = l1 - l0 + 1;
+        // compensated (Kahan) sums: what a window gains and loses leaves no drift
+        float2 g = make_float2(0.f, 0.f), lost = make_float2(0.f, 0.f);
+        auto add_to = [&](float x, float y) {
+            const float px = x - lost.x, py = y - lost.y;
+            const float nx = g.x + px, ny = g.y + py;
+            lost = make_float2((nx - g.x) - px, (ny - g.y) - py);
+            g = make_float2(nx, ny);
+        };
+        if (lane < L)
+            for (int l = 0; l < nl; ++l) add_to(Pd[l * kBand].x, Pd[l * kBand].y);
+        // row i of R takes the place of the band's row i, which every lane has read then
+        // (row i of the band is the first of those that a later window drops)
+        for (int i = 0; i < L; ++i) {
+            const float2 v = make_float2(g.x * norm, g.y * norm);
+            if (i + 1 + lane < L) {
+                const float2 add = Pd[(nl + i) * kBand], sub = Pd[i * kBand];
+                add_to(add.x - sub.x, add.y - sub.y);
             }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-            last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
-            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
-        }
-        any = __any_sync(0xffffffffu, any);
-        if (!any) {
-            if (lane == 0) out[t] = make_float2(0.f, 0.f);
-            continue;
-        }
-        if (cnt < 2) {
-            if (lane == 0) out[t] = sum;
-            continue;
-        }
-        int L = (int)floorf(a.l_frac * (float)cnt);
-        L = max(1, min(L, cnt - 1));
-        if (last - L + 1 < first) {  // no subarray fits: plain sum
-            if (lane == 0) out[t] = sum;
-            continue;
-        }
-        const int l0 = first, l1 = last - L + 1;  // subarray starts
-        // R = sum over rows of the depth window
-        for (int i = lane; i < L * (kLMax + 1); i += 32) (&R[0][0])[i] = make_float2(0.f, 0.f);
-        const int64_t r0 = max((int64_t)0, iz - a.K), r1 = min(a.nz - 1, iz + a.K);
-        for (int64_t r = r0; r <= r1; ++r) {
             __syncwarp();
-            for (int c = lane; c < M; c += 32) row[c] = __ldg(base + (int64_t)c * P + ix * a.nz + r);
-            __syncwarp();
-            const int d = lane;
-            if (d < L) {
-                float2 g = make_float2(0.f, 0.f);  // G(0, d)
-                for (int l = l0; l <= l1; ++l) {
-                    const float2 q = cmul_conj(row[l], row[l + d]);
-                    g.x += q.x;
-                    g.y += q.y;
-                }
-                for (int i = 0; i + d < L; ++i) {
-                    R[i][i + d].x += g.x;
-                    R[i][i + d].y += g.y;
-                    if (i + 1 + d < L) {  // slide to G(i+1, i+1+d)
-                        const float2 add = cmul_conj(row[l1 + i + 1], row[l1 + i + 1 + d]);
-                        const float2 sub = cmul_conj(row[l0 + i], row[l0 + i + d]);
-                        g.x += add.x - sub.x;
-                        g.y += add.y - sub.y;
-                    }
-                }
-            }
+            if (i + lane < L) band[i * kBand + i + lane] = v;
         }
-        __syncwarp();
-        // normalise, mirror to the lower triangle, forward-backward, diagonal loading
-        const float norm = 1.f / ((float)(2 * a.K + 1) * (float)(cnt - L + 1));
-        for (int idx = lane; idx < L * L; idx += 32) {
-            const int i = idx / L, j = idx - (idx / L) * L;
-            if (j >= i) {
-                R[i][j].x *= norm;
-                R[i][j].y *= norm;
-            }
-        }
-        __syncwarp();
+    }
+    float2 (*R)[kBand] = reinterpret_cast<float2 (*)[kBand]>(band);
+    __syncwarp();
+    if (a.fb) {
+        // (J conj(R) J)[i][j] = conj(R[L-1-i][L-1-j]); average the upper triangle
         for (int idx = lane; idx < L * L; idx += 32) {
             const int i = idx / L, j = idx - (idx / L) * L;
             if (j < i) R[i][j] = make_float2(R[j][i].x, -R[j][i].y);
         }
         __syncwarp();
-        if (a.fb) {
-            // (J conj(R) J)[i][j] = conj(R[L-1-i][L-1-j]); average the upper triangle
-            float2 nv[kLMax];
-            int n = 0;
-            for (int idx = lane; idx < L * L; idx += 32, ++n) {
-                const int i = idx / L, j = idx - (idx / L) * L;
-                const float2 q = R[L - 1 - i][L - 1 - j];
-                nv[n] = make_float2(0.5f * (R[i][j].x + q.x), 0.5f * (R[i][j].y - q.y));
-            }
-            __syncwarp();
-            n = 0;
-            for (int idx = lane; idx < L * L; idx += 32, ++n) {
-                const int i = idx / L, j = idx - (idx / L) * L;
-                R[i][j] = nv[n];
-            }
-            __syncwarp();
-        }
-        float tr = lane < L ? R[lane][lane].x : 0.f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
-        if (lane < L) R[lane][lane].x += a.reg / (float)L * tr;
-        __syncwarp();
-        // Cholesky R = U^H U (U upper, over R's upper triangle)
-        for (int k = 0; k < L; ++k) {
-            float dkk = R[k][k].x;
-            for (int m = 0; m < k; ++m) dkk -= R[m][k].x * R[m][k].x + R[m][k].y * R[m][k].y;
-            const float ukk = sqrtf(fmaxf(dkk, 1e-30f));
-            const int j = lane;
-            float2 ukj = make_float2(0.f, 0.f);
-            if (j > k && j < L) {
-                float2 s = R[k][j];
-                for (int m = 0; m < k; ++m) {
-                    const float2 q = cmul_conj(R[m][k], R[m][j]);
-                    s.x -= q.x;
-                    s.y -= q.y;
-                }
-                ukj = make_float2(s.x / ukk, s.y / ukk);
-            }
-            __syncwarp();
-            if (j > k && j < L) R[k][j] = ukj;
-            if (lane == 0) R[k][k] = make_float2(ukk, 0.f);
-            __syncwarp();
-        }
-        // U^H y = 1 (forward), U x = y (backward); v holds y then x
-        if (lane == 0) {
-            for (int i = 0; i < L; ++i) {
-                float2 s = make_float2(1.f, 0.f);
-                for (int m = 0; m < i; ++m) {  // (U^H)[i][m] = conj(U[m][i])
-                    const float2 q = cmul_conj(R[m][i], v[m]);
-                    s.x -= q.x;
-                    s.y -= q.y;
-                }
-                v[i] = make_float2(s.x / R[i][i].x, s.y / R[i][i].x);
-            }
-            for (int i = L - 1; i >= 0; --i) {
-                float2 s = v[i];
-                for (int m = i + 1; m < L; ++m) {
-                    const float2 u = R[i][m], x = v[m];
-                    s.x -= u.x * x.x - u.y * x.y;
-                    s.y -= u.x * x.y + u.y * x.x;
-                }
-                v[i] = make_float2(s.x / R[i][i].x, s.y / R[i][i].x);
-            }
+        float2 nv[kLMax];
+        int n = 0;
+        for (int idx = lane; idx < L * L; idx += 32, ++n) {
+            const int i = idx / L, j = idx - (idx / L) * L;
+            const float2 q = R[L - 1 - i][L - 1 - j];
+            nv[n] = make_float2(0.5f * (R[i][j].x + q.x), 0.5f * (R[i][j].y - q.y));
         }
         __syncwarp();
-        // w = x / (1^T x); z = sum_l sum_i conj(w_i) conj(x_iz[l + i]) * Ma / (Ma - L + 1)
-        float2 den = lane < L ? v[lane] : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            den.x += __shfl_xor_sync(0xffffffffu, den.x, o);
-            den.y += __shfl_xor_sync(0xffffffffu, den.y, o);
-        }
-        // the pixel's own row
-        for (int c = lane; c < M; c += 32) row[c] = __ldg(base + (int64_t)c * P + p);
-        __syncwarp();
-        float2 z = make_float2(0.f, 0.f);
-        if (lane < L) {
-            const float dd = den.x * den.x + den.y * den.y;
-            const float2 xi = v[lane];
-            const float2 w = make_float2((xi.x * den.x + xi.y * den.y) / dd, (xi.y * den.x - xi.x * den.y) / dd);
-            for (int l = l0; l <= l1; ++l) {
-                const float2 x = row[l + lane];
-                // conj(w) * conj(x) = conj(w * x)
-                z.x += w.x * x.x - w.y * x.y;
-                z.y -= w.x * x.y + w.y * x.x;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
-            z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
-        }
-        if (lane == 0) {
-            const float sc = (float)cnt / (float)(cnt - L + 1);
-            out[t] = make_float2(z.x * sc, z.y * sc);
+        n = 0;
+        for (int idx = lane; idx < L * L; idx += 32, ++n) {
+            const int i = idx / L, j = idx - (idx / L) * L;
+            R[i][j] = nv[n];
         }
         __syncwarp();
     }
+    float tr = lane < L ? R[lane][lane].x : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    // ---- Cholesky R = U^H U, lane j column j, four rows at a time, and U^H y = 1 ----
+    // (rolled loops: unrolled over all rows with the column in registers, the warps of an SM
+    // waited for instructions)
+    const float load = a.reg / (float)L * tr;
+    float2 y = make_float2(lane < L ? 1.f : 0.f, 0.f);
+    float inv_diag = 0.f;
+    for (int k0 = 0; k0 < L; k0 += 4) {
+        float2 s[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            s[r] = k0 + r <= lane && lane < L ? R[k0 + r][lane] : make_float2(0.f, 0.f);
+            if (k0 + r == lane) s[r].x += load;
+        }
+        auto take = [](float2& v, float2 c, float2 u) {  // v -= conj(c) u
+            v.x = fmaf(-c.x, u.x, fmaf(-c.y, u.y, v.x));
+            v.y = fmaf(-c.x, u.y, fmaf(c.y, u.x, v.y));
+        };
+#pragma unroll 2
+        for (int m = 0; m < k0; ++m) {
+            const float2 u = R[m][lane];
+            const float4 c0 = *reinterpret_cast<const float4*>(&R[m][k0]), c1 = *reinterpret_cast<const float4*>(&R[m][k0 + 2]);
+            take(s[0], make_float2(c0.x, c0.y), u);
+            take(s[1], make_float2(c0.z, c0.w), u);
+            take(s[2], make_float2(c1.x, c1.y), u);
+            take(s[3], make_float2(c1.z, c1.w), u);
+        }
+        __syncwarp();  // R's rows k0 .. k0 + 3 are read: U's take their place
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int k = k0 + r;
+            if (k >= L) continue;
+            const float inv = 1.f / sqrtf(fmaxf(__shfl_sync(0xffffffffu, s[r].x, k), 1e-30f));
+            const float2 u = lane > k && lane < L ? make_float2(s[r].x * inv, s[r].y * inv) : make_float2(0.f, 0.f);
+            R[k][lane] = u;
+            if (lane == k) {
+                inv_diag = inv;
+                y = make_float2(y.x * inv, y.y * inv);
+            }
+            take(y, u, shfl2(y, k));
+#pragma unroll
+            for (int q = r + 1; q < 4; ++q) take(s[q], shfl2(u, (k0 + q) & 31), u);
+        }
+        __syncwarp();
+    }
+    // ---- U x = y, then w = x / (1^T x) ----
+    for (int m = L - 1; m >= 0; --m) {
+        if (lane == m) y = make_float2(y.x * inv_diag, y.y * inv_diag);
+        const float2 x = shfl2(y, m);
+        if (lane < m) {
+            const float2 u = R[lane][m];
+            y.x -= u.x * x.x - u.y * x.y;
+            y.y -= u.x * x.y + u.y * x.x;
+        }
+    }
+    float2 den = lane < L ? y : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        den.x += __shfl_xor_sync(0xffffffffu, den.x, o);
+        den.y += __shfl_xor_sync(0xffffffffu, den.y, o);
+    }
+    // z = sum_i conj(w_i) sum_l conj(x_iz[l + i]) * Ma / (Ma - L + 1)
+    float2 z = make_float2(0.f, 0.f);
+    if (lane < L) {
+        const float dd = den.x * den.x + den.y * den.y;
+        const float2 w = make_float2((y.x * den.x + y.y * den.y) / dd, (y.y * den.x - y.x * den.y) / dd);
+        float2 s = make_float2(0.f, 0.f);
+        for (int l = l0; l <= l1; ++l) {
+            s.x += own[l + lane].x;
+            s.y += own[l + lane].y;
+        }
+        z = make_float2(w.x * s.x - w.y * s.y, -(w.x * s.y + w.y * s.x));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
+        z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
+    }
+    const float sc = (float)cnt / (float)(cnt - L + 1);
+    return make_float2(z.x * sc, z.y * sc);
 }
 
+__global__ void __launch_bounds__(32 * kWarps, 2) capon_kernel(const float2* __restrict__ cube,
+                                                               const float* __restrict__ apod, float2* __restrict__ out,
+                                                               const CaponArgs a) {
+    extern __shared__ __align__(16) float smem[];
+    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int M = (int)a.M;
+    float* rows = smem + wi * warp_words(M);
+    float2* band = reinterpret_cast<float2*>(rows + band_offset(M));
+    float2* own = reinterpret_cast<float2*>(rows + own_offset(M));
+    const int64_t P = a.nz * a.nx;
+    const int64_t per_col = (a.nz + a.group - 1) / a.group, total = per_col * a.nx * a.F;
+    for (int64_t t = (int64_t)blockIdx.x * nwarps + wi; t < total; t += (int64_t)gridDim.x * nwarps) {
+        const int64_t f = t / (per_col * a.nx), rest = t - f * per_col * a.nx;
+        const int64_t ix = rest / per_col;
+        const int iz0 = (int)(rest - ix * per_col) * a.group, nz = (int)a.nz;
+        const int np = min(a.group, nz - iz0);                      // this warp's pixels iz0 .. iz0 + np - 1
+        const float2* base = cube + f * a.M * P + ix * a.nz;        // [M][P] at this column's first depth
+        // every pixel's active channels, all-zero test and plain sum of its own row
+        int my_lo = 0, my_hi = 0, my_L = 0, my_cnt = 0;  // lane g: pixel iz0 + g
+        int first = M, last = -1;  // over the pixels that need weights
+        int Lmax = 0;
+#pragma unroll
+        for (int g = 0; g < kGroup; ++g) {
+            if (g >= np) continue;
+            const int64_t p = ix * a.nz + iz0 + g;
+            int lo = M, hi = -1, cnt = 0;
+            bool any = false;
+            float2 sum = make_float2(0.f, 0.f);
+            for (int c = lane; c < M; c += 32) {
+                const float2 x = __ldg(base + (int64_t)c * P + iz0 + g);
+                any |= hypotf(x.x, x.y) > 2.220446049250313e-16f;
+                sum.x += x.x;
+                sum.y += x.y;
+                if (fabsf(__ldg(apod + (int64_t)c * P + p)) > a.crit) {
+                    lo = min(lo, c);
+                    hi = max(hi, c);
+                    ++cnt;
+                }
+            }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+                sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+            }
+            any = __any_sync(0xffffffffu, any);
+            int L = (int)floorf(a.l_frac * (float)cnt);
+            L = max(1, min(L, cnt - 1));
+            if (!any || cnt < 2 || hi - L + 1 < lo) {  // silent: 0; no subarray fits: the plain sum
+                if (lane == 0) out[f * P + p] = any ? sum : make_float2(0.f, 0.f);
+                continue;
+            }
+            if (lane == g) {
+                my_lo = lo;
+                my_hi = hi;
+                my_L = L;
+                my_cnt = cnt;
+            }
+            first = min(first, lo);
+            last = max(last, hi);
+            Lmax = max(Lmax, L);
+        }
+        if (Lmax == 0) continue;
+
+        // ---- the band of the Gram matrix over the rows that every pixel's window shares ----
+        const int r0 = max(0, iz0 + np - 1 - a.K), r1 = min(nz - 1, iz0 + a.K);
+        const int fb = first / kTileC, nblk = last / kTileC - fb + 1, c0 = fb * kTileC;
+        const int wide = (Lmax + kTileC - 2) / kTileC + 1;  // tiles of one block row that reach d < L
+        int ntiles = 0;
+        for (int i = 0; i < nblk; ++i) ntiles += min(wide, nblk - i);
+        // rows [ra, rb) (at most kRows) of the staged channels; kRows neighbouring rows of 4
+        // channels per load; channels past M are zeros
+        auto stage = [&](int ra, int nr) {
+            __syncwarp();
+            const int r = lane % kRows;
+            const float2* src = base + (int64_t)c0 * P + ra + r;
+            for (int c = lane / kRows; c < nblk * kTileC; c += 32 / kRows) {
+                float2 x = make_float2(0.f, 0.f);
+                if (r < nr && c0 + c < M) x = __ldg(src + (int64_t)c * P);
+                float* dst = rows + (r * nblk + c / kTileC) * kTileStride + c % kTileC;
+                dst[0] = x.x;
+                dst[kTileC] = x.y;
+            }
+            __syncwarp();
+        };
+        for (int tb = 0; tb < ntiles; tb += 32) {  // more than one pass only for single pixels
+            int ti = 0, tj = tb + lane;  // this lane's tile (block row ti, block column tj)
+            const bool mine = tj < ntiles;
+            if (!mine) tj = 0;
+            while (tj >= min(wide, nblk - ti)) {
+                tj -= min(wide, nblk - ti);
+                ++ti;
+            }
+            tj += ti;
+            // one staged row's 8 channels of a block: real parts, then imaginary parts
+            auto block_at = [&](int q, int blk) { return rows + (q * nblk + blk) * kTileStride; };
+            auto load8 = [&](const float* src, float (&x)[kTileC], float (&y)[kTileC]) {
+                const float4* v = reinterpret_cast<const float4*>(src);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 p = v[h], q = v[2 + h];
+                    x[4 * h] = p.x; x[4 * h + 1] = p.y; x[4 * h + 2] = p.z; x[4 * h + 3] = p.w;
+                    y[4 * h] = q.x; y[4 * h + 1] = q.y; y[4 * h + 2] = q.z; y[4 * h + 3] = q.w;
+                }
+            };
+            float re[kTileC][kTileC], im[kTileC][kTileC];  // sums of the tile over the common rows
+#pragma unroll
+            for (int u = 0; u < kTileC; ++u)
+#pragma unroll
+                for (int v = 0; v < kTileC; ++v) re[u][v] = im[u][v] = 0.f;
+            for (int rb = r0; rb <= r1; rb += kRows) {
+                const int nr = min(kRows, r1 - rb + 1);
+                stage(rb, nr);
+                for (int q = 0; q < nr; ++q) {
+                    float bx[kTileC], by[kTileC];
+                    load8(block_at(q, tj), bx, by);
+                    const float4* xa = reinterpret_cast<const float4*>(block_at(q, ti));
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float4 ax4 = xa[h], ay4 = xa[2 + h];
+                        const float ax[4] = {ax4.x, ax4.y, ax4.z, ax4.w}, ay[4] = {ay4.x, ay4.y, ay4.z, ay4.w};
+#pragma unroll
+                        for (int w = 0; w < 4; ++w)
+#pragma unroll
+                            for (int v = 0; v < kTileC; ++v) {  // += conj(a) b
+                                const int u = 4 * h + w;
+                                re[u][v] = fmaf(ax[w], bx[v], fmaf(ay[w], by[v], re[u][v]));
+                                im[u][v] = fmaf(ax[w], by[v], fmaf(-ay[w], bx[v], im[u][v]));
+                            }
+                    }
+                }
+            }
+            // ---- each pixel: its own rows besides the common ones, then its weights ----
+            for (int g = 0; g < np; ++g) {
+                const int L = __shfl_sync(0xffffffffu, my_L, g);
+                if (L == 0) continue;
+                const int below = r0 - max(0, iz0 + g - a.K), above = min(nz - 1, iz0 + g + a.K) - r1;  // own rows
+                if (below > 0) stage(r0 - below, below);
+                __syncwarp();  // (no own row: the pixel before has read the band)
+                auto own_rows = [&](int n, int u, float (&tx)[kTileC], float (&ty)[kTileC]) {
+                    for (int q = 0; q < n; ++q) {
+                        float bx[kTileC], by[kTileC];
+                        load8(block_at(q, tj), bx, by);
+                        const float ax = block_at(q, ti)[u], ay = block_at(q, ti)[kTileC + u];
+#pragma unroll
+                        for (int v = 0; v < kTileC; ++v) {
+                            tx[v] = fmaf(ax, bx[v], fmaf(ay, by[v], tx[v]));
+                            ty[v] = fmaf(ax, by[v], fmaf(-ay, bx[v], ty[v]));
+                        }
+                    }
+                };
+                // `above` rows are staged behind the `below` ones: together at most kGroup - 1
+                if (above > 0) {
+                    const int r = lane % kRows;
+                    for (int c = lane / kRows; c < nblk * kTileC; c += 32 / kRows) {
+                        if (r >= above) continue;
+                        float2 x = make_float2(0.f, 0.f);
+                        if (c0 + c < M) x = __ldg(base + (int64_t)(c0 + c) * P + r1 + 1 + r);
+                        float* dst = rows + ((below + r) * nblk + c / kTileC) * kTileStride + c % kTileC;
+                        dst[0] = x.x;
+                        dst[kTileC] = x.y;
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int u = 0; u < kTileC; ++u) {
+                    float tx[kTileC], ty[kTileC];
+#pragma unroll
+                    for (int v = 0; v < kTileC; ++v) {
+                        tx[v] = re[u][v];
+                        ty[v] = im[u][v];
+                    }
+                    own_rows(below + above, u, tx, ty);
+#pragma unroll
+                    for (int v = 0; v < kTileC; ++v) {
+                        const int d = (tj - ti) * kTileC + v - u;
+                        if (mine && d >= 0 && d < L) band[(ti * kTileC + u) * kBand + d] = make_float2(tx[v], ty[v]);
+                    }
+                }
+                if (tb + 32 < ntiles) continue;  // the band is not complete yet
+                const int cnt = __shfl_sync(0xffffffffu, my_cnt, g), l0 = __shfl_sync(0xffffffffu, my_lo, g);
+                const int l1 = __shfl_sync(0xffffffffu, my_hi, g) - L + 1;  // subarray starts l0 .. l1
+                for (int c = lane; c < M; c += 32) own[c] = __ldg(base + (int64_t)c * P + iz0 + g);
+                __syncwarp();
+                const float2 z = capon_value(band, own, a, lane, L, cnt, l0 - c0, l0, l1);
+                if (lane == 0) out[f * P + ix * a.nz + iz0 + g] = z;
+                __syncwarp();
+            }
+        }
+    }
+}
 }  // namespace
 
 extern "C" int ustb_capon(const void* cube, const float* apodization, int64_t nz, int64_t nx, int64_t M, int64_t F,
@@ -268,11 +434,25 @@ extern "C" int ustb_capon(const void* cube, const float* apodization, int64_t nz
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t total = nz * nx * F;
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + kWarps - 1) / kWarps,
+    // neighbouring pixels per warp: they share 2K + 2 - g rows of the Gram matrix and add
+    // g - 1 of their own each, so the rows per pixel are (2K + 2 - g) / g + g - 1; a band of
+    // more than 64 channels takes several passes of tiles, which groups cannot keep
+    a.group = 1;
+    if (M <= 64) {
+        auto rows_of = [&](int g) { return (double)(2 * K_samples + 2 - g) / g + g - 1; };
+        for (int g = 2; g <= std::min(kGroup, 2 * K_samples + 1); ++g)
+            if (rows_of(g) < rows_of(a.group)) a.group = g;
+    }
+    const int64_t total = (nz + a.group - 1) / a.group * nx * F;
+    // as many pixels (warps) per CTA as leave room for two CTAs per SM
+    const int per_warp = warp_words((int)M) * (int)sizeof(float);
+    const int warps = std::max(1, std::min(kWarps, 110 * 1024 / per_warp));
+    const size_t smem = (size_t)warps * per_warp;
+    USTB_CUDA(cudaFuncSetAttribute(capon_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + warps - 1) / warps,
                                                                           (int64_t)sms * 64));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    capon_kernel<<<grid, 32 * kWarps, 0, s>>>(static_cast<const float2*>(cube), apodization,
+    capon_kernel<<<grid, 32 * warps, smem, s>>>(static_cast<const float2*>(cube), apodization,
                                               static_cast<float2*>(out), a);
     USTB_CUDA(cudaGetLastError());
     return USTB_OK;
