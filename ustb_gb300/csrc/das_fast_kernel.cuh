@@ -45,6 +45,7 @@
 #include <type_traits>
 
 #include "das_fast.cuh"
+#include "f32x2.cuh"
 #include "phasor.cuh"
 
 namespace ustb {
@@ -202,39 +203,6 @@ __device__ __forceinline__ void block_min(float (&v)[NV], int* red) {
         const int m = __shfl_sync(0xffffffffu, mine, i);
         v[i] = __int_as_float(m ^ ((m >> 31) & 0x7fffffff));
     }
-}
-
-// ---- two floats per instruction (packed FP32 pairs) ----------------------------------
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2_rz(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
 }
 
 template <bool CPLX>
