@@ -13,8 +13,10 @@
 // values in registers) and channels inner (rx values re-read once per chunk);
 // for .transmit/.none, channels outer and wave chunks inner.
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "phasor.cuh"
 
 namespace {
@@ -66,6 +68,13 @@ __device__ __forceinline__ void store(const TableArgs& A, int64_t idx, int64_t f
 // multiplied by zero, so non-finite samples behave as in das_c, which skips
 // those units).  All WC sample loads are then in flight together.
 constexpr int WC = 8;
+// At most this many waves run in chunks of channels (das_table_few_waves), where those were
+// the faster ones (128 channels, 200 x 200 pixels, chunks of waves against chunks of
+// channels, us; real data crosses at the same counts):
+//   both      1 wave 75 / 42, 2 waves 71 / 61, 3 waves 72 / 87
+//   receive   1 wave 65 / 27, 3 waves 73 / 69, 4 waves 75 / 91
+//   transmit  1 wave 99 / 35, 5 waves 116 / 96, 8 waves 133 / 141
+constexpr int few_waves(int mode) { return mode == USTB_DIM_BOTH ? 2 : mode == USTB_DIM_RECEIVE ? 3 : 5; }
 
 // A table value that is read once per wave chunk: kept out of L1 so that it does not
 // evict the channel-data lines the sample gathers reuse.
@@ -116,7 +125,11 @@ __device__ __forceinline__ void prefetch_units(const TableArgs& A, IDX nL, const
 // pf: also prefetch into L1 the next channel's sample line of each unit, at this unit's
 // sample index shifted by dn, the receive-delay step to the next channel in samples
 // (clamped into the trace; only where the lines are, not which units are valid).
-template <bool CPLX, int FC, bool PER_WAVE, int NACC, typename IDX, bool MAGIC>
+// PACK: the position and phase arithmetic of two units per instruction.  2 % faster for
+// complex chunks of waves (IQ compounding 1.240 -> 1.197 ms) and chunks of channels (one
+// wave, receive kept: 32 -> 26 us); slower where chunks of waves are inner (real RF, 16
+// waves, channels kept: 185 -> 205 us), so not used there.
+template <bool CPLX, int FC, bool PER_WAVE, int NACC, typename IDX, bool MAGIC, bool PACK>
 __device__ __forceinline__ void chunk_units(const TableArgs& A, IDX nL, const IDX* wbase, int wc, int64_t f0,
                                             int nf, const float* txd, const float* txa, float rxd, float rxa,
                                             Acc<CPLX, FC>* acc, bool pf = false, int dn = 0) {
@@ -124,13 +137,7 @@ __device__ __forceinline__ void chunk_units(const TableArgs& A, IDX nL, const ID
     IDX base[WC];
     bool ok[WC];
     const int Lm1 = (int)(A.L - 1);
-#pragma unroll
-    for (int k = 0; k < WC; ++k) {
-        const float delay = __fadd_rn(txd[k], rxd);
-        const float apo = __fmul_rn(txa[k], rxa);
-        const float denay = __fmul_rn(__fsub_rn(delay, A.t0), A.fs);
-        float fl;
-        const int n0 = trunc_floor<MAGIC>(denay, fl);
+    auto place = [&](int k, int n0) {  // validity, prefetch and sample offset of unit k
         ok[k] = k < wc && txa[k] != 0.0f && rxa != 0.0f && n0 > 0 && n0 < Lm1;
         if (pf && k < wc) {
             const int m = min(max(n0 + dn, 1), Lm1 - 1);
@@ -138,17 +145,52 @@ __device__ __forceinline__ void chunk_units(const TableArgs& A, IDX nL, const ID
                             (size_t)(nL + (IDX)A.L + wbase[k] + (IDX)m) * (CPLX ? 8 : 4);
             asm volatile("prefetch.global.L1 [%0];\n" ::"l"(x));
         }
-        b[k] = __fsub_rn(denay, fl);
-        a[k] = __fsub_rn(1.0f, b[k]);
         base[k] = nL + wbase[k] + (IDX)(ok[k] ? n0 : 1);
-        if (CPLX) {
-            float c, s;
-            ustb::expi_reduced(__fmul_rn(A.wd, delay), c, s);
-            wr[k] = c * apo;
-            wi[k] = s * apo;
-        } else {
-            wr[k] = apo;
-            wi[k] = 0.f;
+    };
+    if constexpr (PACK && MAGIC) {
+        using namespace ustb;
+        const f32x2 rxd2 = pack2(rxd, rxd), rxa2 = pack2(rxa, rxa), magic = pack2(8388608.0f, 8388608.0f);
+#pragma unroll
+        for (int k = 0; k < WC; k += 2) {
+            const f32x2 delay = add2(pack2(txd[k], txd[k + 1]), rxd2);
+            const f32x2 apo = mul2(pack2(txa[k], txa[k + 1]), rxa2);
+            const f32x2 denay = mul2(sub2(delay, pack2(A.t0, A.t0)), pack2(A.fs, A.fs));
+            const f32x2 t = add2_rz(denay, magic);  // trunc_floor
+            const f32x2 bb = sub2(denay, sub2(t, magic));
+            const float2 tt = unpack2(t), b2 = unpack2(bb), a2 = unpack2(sub2(pack2(1.0f, 1.0f), bb));
+            place(k, __float_as_int(tt.x) - 0x4B000000);
+            place(k + 1, __float_as_int(tt.y) - 0x4B000000);
+            b[k] = b2.x; b[k + 1] = b2.y;
+            a[k] = a2.x; a[k + 1] = a2.y;
+            float2 w0 = unpack2(apo), w1 = make_float2(0.f, 0.f);
+            if (CPLX) {
+                float2 c, sn;
+                expi_reduced2(mul2(pack2(A.wd, A.wd), delay), c, sn);
+                w1 = unpack2(mul2(pack2(sn.x, sn.y), apo));
+                w0 = unpack2(mul2(pack2(c.x, c.y), apo));
+            }
+            wr[k] = w0.x; wr[k + 1] = w0.y;
+            wi[k] = w1.x; wi[k + 1] = w1.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < WC; ++k) {
+            const float delay = __fadd_rn(txd[k], rxd);
+            const float apo = __fmul_rn(txa[k], rxa);
+            const float denay = __fmul_rn(__fsub_rn(delay, A.t0), A.fs);
+            float fl;
+            place(k, trunc_floor<MAGIC>(denay, fl));
+            b[k] = __fsub_rn(denay, fl);
+            a[k] = __fsub_rn(1.0f, b[k]);
+            if (CPLX) {
+                float c, s;
+                ustb::expi_reduced(__fmul_rn(A.wd, delay), c, s);
+                wr[k] = c * apo;
+                wi[k] = s * apo;
+            } else {
+                wr[k] = apo;
+                wi[k] = 0.f;
+            }
         }
     }
 #pragma unroll
@@ -331,7 +373,7 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
                             continue;
                         }
                         const int dn = __float2int_rn(__fmul_rn(__fsub_rn(rxd1, rxd), A.fs));
-                        chunk_units<CPLX, FC, PER_WAVE, NACC, IDX, MAGIC>(A, nL, wbase, wc, f0, nf, txd, txa, rxd, rxa,
+                        chunk_units<CPLX, FC, PER_WAVE, NACC, IDX, MAGIC, true>(A, nL, wbase, wc, f0, nf, txd, txa, rxd, rxa,
                                                                           acc, pf, dn);
                     }
                 } else {
@@ -375,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
 #pragma unroll
                         for (int k = 0; k < WC; ++k) acc[k].zero();
                     if (rxa != 0.0f)
-                        chunk_units<CPLX, FC, PER_WAVE, NACC, IDX, MAGIC>(A, (IDX)(A.L * n), wbase, wc, f0, nf, txd, txa, rxd,
+                        chunk_units<CPLX, FC, PER_WAVE, NACC, IDX, MAGIC, false>(A, (IDX)(A.L * n), wbase, wc, f0, nf, txd, txa, rxd,
                                                                    rxa, acc);
                     if (MODE == USTB_DIM_NONE)
 #pragma unroll
@@ -388,15 +430,107 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
     }
 }
 
+// Few waves: the chunks of WC units run over channels instead, so that a single wave fills
+// them too (chunks of waves would evaluate WC units for the one).  The roles of the tables
+// are swapped in chunk_units (delays and weights add and multiply in either order): the
+// channels' values are the chunk's, the wave's the common one.  The next chunk's receive
+// values are loaded a chunk ahead.
+template <int MODE, bool CPLX, int FC, typename IDX, bool MAGIC>
+__global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs A) {
+    const int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (p >= A.P) return;
+    const int64_t P = A.P;
+    const int N = (int)A.N, W = (int)A.W;
+    constexpr bool PER_CHANNEL = (MODE == USTB_DIM_TRANSMIT || MODE == USTB_DIM_NONE);
+    Acc<CPLX, FC> acc[PER_CHANNEL ? WC : 1];
+    float rxd[WC], rxa[WC];
+    IDX nbase[WC];
+    auto load_rx = [&](int n0, float* d, float* a) {
+#pragma unroll
+        for (int k = 0; k < WC; ++k) {
+            const bool in = n0 + k < N;
+            a[k] = in ? ld_stream(A.apo_rx + P * (n0 + k) + p) : 0.f;
+            d[k] = in ? ld_stream(A.d_rx + P * (n0 + k) + p) : 0.f;
+        }
+    };
+    for (int64_t f0 = 0; f0 < A.F; f0 += FC) {
+        const int nf = (int)min((int64_t)FC, A.F - f0);
+        // one chunk of channels from n0 on with wave w
+        auto units = [&](int n0, int w, const float* d, const float* a) {
+            const float txd = __ldg(A.d_tx + P * w + p), txa = __ldg(A.apo_tx + P * w + p);
+            if (txa == 0.0f) return;
+            chunk_units<CPLX, FC, PER_CHANNEL, (PER_CHANNEL ? WC : 1), IDX, MAGIC, true>(
+                A, (IDX)(A.LN * w), nbase, min(WC, N - n0), f0, nf, d, a, txd, txa, acc);
+        };
+        auto chunk = [&](int n0) {
+            bool any = false;
+#pragma unroll
+            for (int k = 0; k < WC; ++k) {
+                any |= rxa[k] != 0.0f;
+                nbase[k] = (IDX)(A.L * min(n0 + k, N - 1) + f0 * A.LNW);
+            }
+            return any;
+        };
+        if (MODE == USTB_DIM_RECEIVE) {
+            for (int w = 0; w < W; ++w) {
+                acc[0].zero();
+                for (int n0 = 0; n0 < N; n0 += WC) {
+                    load_rx(n0, rxd, rxa);
+                    if (chunk(n0)) units(n0, w, rxd, rxa);
+                }
+                store<CPLX, FC>(A, p + A.w_f * w, f0, nf, acc[0]);
+            }
+        } else if (MODE == USTB_DIM_BOTH) {
+            acc[0].zero();
+            float d1[WC], a1[WC];
+            load_rx(0, d1, a1);
+            for (int n0 = 0; n0 < N; n0 += WC) {
+#pragma unroll
+                for (int k = 0; k < WC; ++k) {
+                    rxd[k] = d1[k];
+                    rxa[k] = a1[k];
+                }
+                load_rx(n0 + WC, d1, a1);
+                if (!chunk(n0)) continue;
+                for (int w = 0; w < W; ++w) units(n0, w, rxd, rxa);
+            }
+            store<CPLX, FC>(A, p, f0, nf, acc[0]);
+        } else {
+            for (int n0 = 0; n0 < N; n0 += WC) {
+                load_rx(n0, rxd, rxa);
+                const bool any = chunk(n0);
+                auto put = [&](int64_t o) {
+#pragma unroll
+                    for (int k = 0; k < WC; ++k)
+                        if (n0 + k < N) store<CPLX, FC>(A, p + A.rx_f * (n0 + k) + o, f0, nf, acc[k]);
+                };
+#pragma unroll
+                for (int k = 0; k < WC; ++k) acc[PER_CHANNEL ? k : 0].zero();
+                for (int w = 0; w < W; ++w) {
+                    if (any) units(n0, w, rxd, rxa);
+                    if (MODE == USTB_DIM_NONE) {
+                        put(A.w_f * w);
+#pragma unroll
+                        for (int k = 0; k < WC; ++k) acc[PER_CHANNEL ? k : 0].zero();
+                    }
+                }
+                if (MODE == USTB_DIM_TRANSMIT) put(0);
+            }
+        }
+    }
+}
+
 template <int MODE, bool CPLX, typename IDX, bool MAGIC>
 void launch_idx(const TableArgs& A, cudaStream_t s) {
     const unsigned grid = (unsigned)((A.P + kThreads - 1) / kThreads);
-    if (A.F == 1)
-        das_table_kernel<MODE, CPLX, 1, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
-    else if (A.F == 2)
-        das_table_kernel<MODE, CPLX, 2, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
-    else
-        das_table_kernel<MODE, CPLX, 4, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
+    auto start = [&](auto fc) {
+        constexpr int FC = decltype(fc)::value;
+        if (A.W <= few_waves(MODE)) das_table_few_waves<MODE, CPLX, FC, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
+        else das_table_kernel<MODE, CPLX, FC, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
+    };
+    if (A.F == 1) start(std::integral_constant<int, 1>{});
+    else if (A.F == 2) start(std::integral_constant<int, 2>{});
+    else start(std::integral_constant<int, 4>{});
 }
 
 // 32-bit sample indices when every index of the call (and one past it) fits 31 bits;

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include "f32x2.cuh"
+
 namespace ustb {
 
 // 2*pi split in two floats (Cody & Waite additive range reduction): C1 is
@@ -25,6 +27,15 @@ __device__ __forceinline__ void expi_reduced(float x, float& c, float& s) {
     float r = fmaf(-k, kTwoPiHi, x);
     r = fmaf(-k, kTwoPiLo, r);
     __sincosf(r, &s, &c);
+}
+
+// Two of them, in the same roundings.
+__device__ __forceinline__ void expi_reduced2(f32x2 x, float2& c, float2& s) {
+    const f32x2 big = pack2(12582912.0f, 12582912.0f);
+    const f32x2 nk = sub2(big, fma2(x, pack2(kInvTwoPi, kInvTwoPi), big));  // -k
+    const float2 r = unpack2(fma2(nk, pack2(kTwoPiLo, kTwoPiLo), fma2(nk, pack2(kTwoPiHi, kTwoPiHi), x)));
+    __sincosf(r.x, &s.x, &c.x);
+    __sincosf(r.y, &s.y, &c.y);
 }
 
 }  // namespace ustb

@@ -52,17 +52,14 @@ def channel_tensor(data, device) -> torch.Tensor:
 
 
 def hilbert_last(x: torch.Tensor) -> torch.Tensor:
-    """Analytic signal along the last dimension (the FFT method of MATLAB's hilbert)."""
+    """Analytic signal along the last dimension (the FFT method of MATLAB's hilbert): the
+    positive frequencies doubled and the negative ones zeroed in place (two launches; a
+    vector of factors costs five)."""
     L = x.shape[-1]
     X = torch.fft.fft(x.to(torch.float32), dim=-1)
-    h = torch.zeros(L, dtype=torch.float32, device=x.device)
-    if L % 2 == 0:
-        h[0] = h[L // 2] = 1.0
-        h[1:L // 2] = 2.0
-    else:
-        h[0] = 1.0
-        h[1:(L + 1) // 2] = 2.0
-    return torch.fft.ifft(X * h, dim=-1).to(torch.complex64).contiguous()
+    X[..., 1:(L + 1) // 2].mul_(2.0)
+    X[..., L // 2 + 1:].zero_()
+    return torch.fft.ifft(X, dim=-1).to(torch.complex64).contiguous()
 
 
 class DAS:
