@@ -46,6 +46,44 @@ int shape_for(int dim, bool cplx, int32_t requested) {
     }
 }
 
+// CTAs (parts) per sub-tile of a grid launch.  Few sub-tiles leave SMs without work or a
+// last round of long CTAs; each part sets the tile up again.  The number taken minimises
+//   (rounds + 1/4) (set-up + stages / parts),
+// rounds of CTAs (two per SM; half a round at least: one CTA per SM) with a quarter for
+// the uneven end, times a CTA's length in stages (its set-up is worth 2 and one for every
+// 128 channels and waves); another part must shorten it by 1.5 %.  Measured, one part
+// against this rule: synthetic aperture of real traces, 128 x 128, 0.640 and 0.591 ms,
+// 115 x 115 on 223 x 73 pixels, 480 and 225 us; a transmit image of 145 channels x 9 waves
+// on 73 x 252 pixels, 97 and 60 us; 75-wave IQ compounding, 525 us either way.
+// transmit and receive split where their outputs do not overlap (the epilogue sums over
+// channels, so it does not split).
+int parts_for(const Params& A, int dim, bool epi, int32_t requested, int& parts) {
+    parts = 1;
+    if (dim == USTB_DIM_BOTH && requested > 0) {
+        parts = requested;
+        return USTB_OK;
+    }
+    if (dim == USTB_DIM_NONE || epi) return USTB_OK;
+    int dev = 0, sms = 0;
+    USTB_CUDA(cudaGetDevice(&dev));
+    USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    constexpr int kCG[3] = {2, 8, 16}, kKW[3] = {16, 4, 2};
+    const int64_t groups = (A.N + kCG[A.shape] - 1) / kCG[A.shape], chunks = (A.W + kKW[A.shape] - 1) / kKW[A.shape];
+    const int64_t most = dim == USTB_DIM_RECEIVE ? chunks : dim == USTB_DIM_TRANSMIT ? groups : groups * chunks;
+    const double stages = (double)groups * (double)chunks;
+    const double setup = 2.0 + (double)(A.N + A.W) / 128.0;  // of a CTA, in stages
+    const double rounds = (double)A.n_tiles * ustb::kSub * (double)A.F / (2.0 * sms);  // of one part each
+    double best = 0.0;
+    for (int k = 1; k <= 8 && k <= most; ++k) {
+        const double cost = (std::max(k * rounds, 0.5) + 0.25) * (setup + stages / k);
+        if (k == 1 || cost < 0.985 * best) {
+            parts = k;
+            best = cost;
+        }
+    }
+    return USTB_OK;
+}
+
 // one stored sample (global memory) as float2
 template <int ST, bool CPLX>
 __device__ __forceinline__ float2 load_sample(const void* ch, int64_t i) {
@@ -130,23 +168,28 @@ int fill_entries(const void* ch, int32_t storage, bool cplx, int64_t L, int64_t 
     return USTB_OK;
 }
 
-// Allocate (stream-ordered, from the library pool) and fill one request's entries.
+// Allocate (stream-ordered, from the library pool) and fill one request's entries.  Behind
+// them (on a 256-byte boundary) lie ``sums`` bytes and ``tickets`` zeroed bytes; *behind
+// points there.
 int build_entries(const void* ch, int32_t storage, bool cplx, int64_t L, int64_t N, int64_t W, int64_t F,
-                  void** out, cudaStream_t s) {
+                  void** out, cudaStream_t s, int64_t sums = 0, int64_t tickets = 0, char** behind = nullptr) {
     *out = nullptr;
-    const int64_t bytes = entry_bytes(L, N, W, F, cplx);
+    const int64_t ent = (entry_bytes(L, N, W, F, cplx) + 255) & ~int64_t(255), bytes = ent + sums + tickets;
     if (bytes == 0) return USTB_OK;
     int dev = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     cudaMemPool_t pool = entry_pool(dev);
     USTB_REQUIRE(pool, USTB_E_CUDA, "could not create the entry memory pool on device %d", dev);
-    const cudaError_t e = cudaMallocFromPoolAsync(out, (size_t)bytes, pool, s);
+    cudaError_t e = cudaMallocFromPoolAsync(out, (size_t)bytes, pool, s);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         *out = nullptr;
         ustb::set_error("%lld bytes of interpolation entries: %s", (long long)bytes, cudaGetErrorString(e));
         return USTB_E_OOM;
     }
+    if (behind) *behind = static_cast<char*>(*out) + ent;
+    // before the entries, so that the beamforming launch follows their kernel
+    if (tickets) USTB_CUDA(cudaMemsetAsync(static_cast<char*>(*out) + ent + sums, 0, (size_t)tickets, s));
     return fill_entries(ch, storage, cplx, L, N, W, F, *out, s);
 }
 
@@ -217,7 +260,9 @@ static int make_params(const void* ch, int32_t storage, int32_t is_complex, int6
     A.fd_fs = (double)A.fd / (double)A.fs;
     A.wave_step = N * A.Lp;
     A.frame_step = W * A.wave_step;
+    A.c = g->sound_speed;
     A.inv_c = 1.f / g->sound_speed;
+    A.fs_c = (double)A.fs / (double)A.c;
     A.lens = g->lens_delay;
     A.rx_window = g->rx_window;
     {
@@ -239,13 +284,18 @@ static int make_params(const void* ch, int32_t storage, int32_t is_complex, int6
     A.rx_f = os.rx_f; A.w_f = os.w_f; A.f_f = os.f_f;
     A.flags = flags;
     USTB_REQUIRE(g->ctas_per_tile >= 0 && g->ctas_per_tile <= 4, USTB_E_ARG, "ctas_per_tile must be 0 to 4");
-    A.split = g->ctas_per_tile;  // 0: chosen at launch
+    A.after_entries = false;
+    A.partial = nullptr;
+    A.tickets = nullptr;
     USTB_REQUIRE(g->stage_shape >= 0 && g->stage_shape <= 3, USTB_E_ARG, "stage_shape must be 0, 1, 2 or 3");
     USTB_REQUIRE(g->stage_shape == 0 || dimension == USTB_DIM_BOTH ||
                      (dimension == USTB_DIM_RECEIVE) == (g->stage_shape == 1),
                  USTB_E_ARG, "stage_shape %d does not fit dimension %d (receive: 1; transmit/none: 2 or 3)",
                  (int)g->stage_shape, (int)dimension);
     A.shape = shape_for(dimension, is_complex != 0, g->stage_shape);
+    A.split = 1;
+    const int rc = parts_for(A, dimension, epilogue != 0, g->ctas_per_tile, A.split);
+    if (rc) return rc;
     A.fpi = 1;
     return USTB_OK;
 }
@@ -261,11 +311,32 @@ extern "C" int ustb_das_fast(const void* ch, int32_t storage, int32_t is_complex
     bool empty = false;
     int rc = make_params(ch, storage, is_complex, L, N, W, F, g, dimension, epilogue, out, flags, s, A, empty);
     if (rc || empty) return rc;
+    // partial sums of split sub-tiles and their tickets behind the entries
+    const int64_t nt = g->n_tiles, nsub = nt * ustb::kSub * F;
+    int64_t sums = 0, tickets = 0;
+    if (dimension == USTB_DIM_BOTH && A.split > 1) {
+        sums = nsub * A.split * ustb::kThreads * (int64_t)sizeof(float2);
+        tickets = nsub * (int64_t)sizeof(unsigned);
+    }
     void* ent = nullptr;
-    rc = build_entries(ch, storage, is_complex != 0, L, N, W, F, &ent, s);
-    if (rc) return rc;
+    char* behind = nullptr;
+    rc = build_entries(ch, storage, is_complex != 0, L, N, W, F, &ent, s, sums, tickets, &behind);
+    if (rc == USTB_E_OOM && tickets) {  // room for the entries alone: whole sub-tiles, or sums in the image
+        tickets = 0;
+        if (g->ctas_per_tile == 0) A.split = 1;
+        ustb::clear_error();
+        rc = build_entries(ch, storage, is_complex != 0, L, N, W, F, &ent, s);
+    }
+    if (rc) {
+        if (ent) (void)cudaFreeAsync(ent, s);
+        return rc;
+    }
     A.entries = ent;
-    const int64_t nt = g->n_tiles;
+    A.after_entries = true;
+    if (tickets) {
+        A.partial = reinterpret_cast<float2*>(behind);
+        A.tickets = reinterpret_cast<unsigned*>(behind + sums);
+    }
     rc = is_complex ? ustb::das_dispatch<true, false>(dimension, epilogue, A.shape, &A, nullptr, 1, nullptr, nt, F, s, 0)
                     : ustb::das_dispatch<false, false>(dimension, 0, A.shape, &A, nullptr, 1, nullptr, nt, F, s, 0);
     const cudaError_t fe = cudaFreeAsync(ent, s);
@@ -306,6 +377,9 @@ extern "C" int ustb_das_fast_entries(const void* entries, int32_t is_complex, in
     if (rc || empty) return rc;
     USTB_REQUIRE(((uintptr_t)entries & 15) == 0, USTB_E_ARG, "entries must be 16-byte aligned");
     A.entries = entries;
+    // no scratch here: the parts of dimension.both add into the image, at most two unless
+    // asked for (two sums are the same in either order)
+    if (dimension == USTB_DIM_BOTH && g->ctas_per_tile == 0) A.split = std::min(A.split, 2);
     const int64_t nt = g->n_tiles;
     return is_complex ? ustb::das_dispatch<true, false>(dimension, epilogue, A.shape, &A, nullptr, 1, nullptr, nt, F, s, 0)
                       : ustb::das_dispatch<false, false>(dimension, 0, A.shape, &A, nullptr, 1, nullptr, nt, F, s, 0);

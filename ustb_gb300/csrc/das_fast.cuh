@@ -7,6 +7,8 @@
 namespace ustb {
 
 constexpr int kTile = USTB_TILE_PIXELS;
+constexpr int kThreads = 256;  // threads of a beamforming CTA
+constexpr int kSub = 2;        // sub-tiles (CTAs) per tile
 
 struct Params {
     const void* entries;  // [F][W][N][Lp] interpolation entries (float4 complex, float2 real)
@@ -20,8 +22,9 @@ struct Params {
     const float* tx_apo_tab;
     const float* rx_apo_tab;
     const float2* pix_phase;
-    float fs, t0, fd, inv_c, lens;
+    float fs, t0, fd, c, inv_c, lens;
     double fd_fs;  // fd / fs
+    double fs_c;   // fs / c
     int64_t wave_step, frame_step;  // entries from a wave (a frame) to the next
     int rx_window;
     float win_r1, win_a, win_e, win_b, win_c, win_d;  // see window_coeffs()
@@ -36,7 +39,10 @@ struct Params {
     float* o_sdmas;
     int64_t rx_f, w_f, f_f;
     uint32_t* flags;
-    int split;  // grid kernel, dimension.both: CTAs per tile (parts of the stage list, 1-4); 0 = auto
+    bool after_entries; // grid kernel: the entries pre-pass is the launch before it
+    int split;          // grid kernel: CTAs (parts) per sub-tile
+    float2* partial;    // dimension.both: sums of the parts [F * sub-tiles][split][kThreads], or null
+    unsigned* tickets;  // parts that have finished, per frame and sub-tile (zeroed)
     int shape;  // stage shape (Shape<> index)
     int fpi;    // persistent kernel: frames per work item (one tile, consecutive frames)
 };

@@ -28,13 +28,18 @@
 // instructions.  Delays relative to the tile bases stay below 80 samples, so j and b
 // keep full sub-sample precision in FP32.
 //
-// What bounds it (75-wave IQ compounding, 400 x 400 pixels, 0.487 ms a launch on a GB300;
+// What bounds it (75-wave IQ compounding, 400 x 400 pixels, 0.49 ms a launch on a GB300;
 // 0.594 ms with one 512-thread CTA per SM and scalar units): the units' 16-byte
 // shared-memory loads alone take 0.24 ms; the stages' copies, barriers and transmit
 // set-ups overlap them only in part.  Measured with parts taken out of a copy: no
 // barriers 0.43 ms, no copies 0.42 ms, no units 0.32 ms.  Not kept, same workload: TMA
 // bulk copies of the windows (0.60 ms: about 50 clocks a copy), three 80-register CTAs
 // per SM with 16-slot stages (0.58 ms), two pixels per thread (0.59 ms: spills).
+// A small launch is bound by setting tiles up, 15,000 clocks of dependent loads and long
+// arithmetic before the first stage (a stage takes about 3,500): the loads are issued
+// together at the start, channels and waves go to different warps, the stage buffers are
+// zeroed meanwhile (32 channels x 1 wave on 135 x 96 pixels: 30 to 26 us a call, with the
+// launch that overlaps the pre-pass's end).
 //
 // Loop orders: waves outer / channels inner for dimension.both and .receive
 // (rx weight per unit, tx weight once per wave chunk); channels outer / waves
@@ -51,8 +56,7 @@
 namespace ustb {
 namespace {
 
-constexpr int kThreads = 256;                   // threads of a CTA: one sub-tile, one pixel per thread
-constexpr int kSub = kTile / kThreads;          // sub-tiles (CTAs) per tile
+static_assert(kTile == kSub * kThreads, "a CTA takes one sub-tile, one pixel per thread");
 constexpr int kBufBytes = 40960;                // a stage buffer: 32 slots x 80 or 16 x 160 complex entries, 32 x 160 real
 constexpr int kItemFrames = 8;                  // frames of a persistent work item at most
 constexpr int kRing = 2;                        // stage buffers: stage s + kRing - 1 is copied during stage s
@@ -222,6 +226,11 @@ __device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
 }
+// The grid may start while the kernel before it in the stream (the entries pre-pass) ends
+// (see launch_dependent): nothing of that kernel is read, and no output written, before
+// this returns.  Every CTA calls it, also one without work.
+__device__ __forceinline__ void wait_for_entries() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Conservative test that channel `n`'s receive window is zero over the whole tile
@@ -317,14 +326,12 @@ __host__ __device__ __forceinline__ TileTables tile_tables(int64_t NP, int64_t W
     return t;
 }
 
-// Once per CTA, before its first tile: zero the stage buffers, so that units with
-// zero weight, which may read past a window's end, never read uninitialised words.
+// Once per CTA: zero the stage buffers, so that units with zero weight, which may read
+// past a window's end, never read uninitialised words.  The caller's barriers follow.
 __device__ __forceinline__ void zero_slots() {
     extern __shared__ __align__(16) unsigned char smem[];
     float4* z = reinterpret_cast<float4*>(smem);
-    for (int i = threadIdx.x; i < (int)(kBuffers / 16); i += blockDim.x)
-        z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
+    for (int i = threadIdx.x; i < (int)(kBuffers / 16); i += kThreads) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 __device__ __forceinline__ float frac_cycles(double v) { return (float)(v - floor(v)); }
@@ -349,8 +356,8 @@ __device__ __forceinline__ float frac_cycles(double v) { return (float)(v - floo
 // after one build of the tile's tables and stage lists (the geometry is the same for
 // every frame of a request).
 template <int MODE, bool CPLX, bool EPI, int SHAPE, bool FRAMES = false>
-__device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int64_t f_first, int half = -1,
-                                         int nfr = 1) {
+__device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int64_t f_first, int part = -1,
+                                         int nfr = 1, bool first = true) {
     constexpr bool ORDER_A = Shape<SHAPE>::WAVES_OUTER;
     static_assert(MODE != USTB_DIM_RECEIVE || ORDER_A, "dimension.receive keeps waves outer");
     static_assert((MODE != USTB_DIM_TRANSMIT && MODE != USTB_DIM_NONE) || !ORDER_A,
@@ -379,23 +386,54 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     __shared__ int s_tx_sph;      // every active wave spherical, and no tx tables
     __shared__ int s_maxn, s_maxw;  // largest active window positions (bits of floats >= 0)
     __shared__ int s_nout, s_nin;
+    __shared__ int s_where[3];      // tile, sub-tile, part: read again after the stages (fewer live registers)
+    __shared__ bool s_last;             // this part is the last of its sub-tile to finish
     __shared__ int s_flat, s_in_plane;  // every element at one z; no elevation offset in the tile
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     const int32_t* tl = A.tiles + (int64_t)tile * kTile;
+    // Setting a tile up is a chain of dependent loads and long-latency arithmetic: what the
+    // tables below read is loaded first, beside the pixel indices and positions, channels
+    // by the first threads and waves by the last ones, so that different warps work on both.
+    const int wtid = kThreads - 1 - tid;
+    float3 next_el = make_float3(0.f, 0.f, 0.f);
+    ustb_wave next_wv = {};
+    auto load_el = [&](int n) {
+        if (n < (int)N) next_el = make_float3(__ldg(A.el + 3 * n), __ldg(A.el + 3 * n + 1), __ldg(A.el + 3 * n + 2));
+    };
+    auto load_wave = [&](int w) {
+        if (w < (int)W) next_wv = A.waves[w];
+    };
+    load_el(tid);
+    load_wave(wtid);
+    const float el0_z = N > 0 ? __ldg(A.el + 2) : 0.f;
     // tile entries outside [0, P) are idle lanes; lane 0 names the tile's anchor pixel
     auto in_image = [&](int32_t q) { return q >= 0 && (int64_t)q < A.P; };
     const int32_t p_own = __ldg(tl + sub * kThreads + tid);
-    const bool live = in_image(p_own);
-    if (!__syncthreads_or(live)) return;  // an idle sub-tile
     const int32_t p_anchor = __ldg(tl);
-    const int64_t p = live ? p_own : (in_image(p_anchor) ? p_anchor : 0);
-    const float px = __ldg(A.px + 3 * p), py = __ldg(A.px + 3 * p + 1), pz = __ldg(A.px + 3 * p + 2);
     // this thread's pixel of the other sub-tile: the delay bases are the whole tile's
     static_assert(kSub == 2, "one other sub-tile");
     const int32_t p_other = __ldg(tl + (sub ^ 1) * kThreads + tid);
-    const bool live_o = in_image(p_other);
+    const bool live = in_image(p_own), live_o = in_image(p_other);
+    if (tid == 0) {
+        s_tx_general = A.tx_apo_tab != nullptr || A.tx_delay_tab != nullptr;
+        s_tx_sph = !s_tx_general;
+        s_maxn = s_maxw = 0;
+        s_flat = 1;
+        s_in_plane = 1;
+        s_where[0] = tile;
+        s_where[1] = sub;
+        s_where[2] = part;
+    }
+    if (first) zero_slots();
+    if (!__syncthreads_or(live)) {  // an idle sub-tile
+        wait_for_entries();
+        return;
+    }
+    const int p = live ? p_own : (in_image(p_anchor) ? p_anchor : 0);
+    const float* const pxyz = A.px + 3 * (int64_t)p;
+    const float px = __ldg(pxyz), py = __ldg(pxyz + 1), pz = __ldg(pxyz + 2);
 
     Box box, tbox;  // sub-tile, whole tile
     {
@@ -422,29 +460,9 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
 
     // ---- per-tile delay bases, window parts, activity and delay/phase coefficients ----
     const double fd_fs = A.fd_fs;
-    if (tid == 0) {
-        s_tx_general = A.tx_apo_tab != nullptr || A.tx_delay_tab != nullptr;
-        s_tx_sph = !s_tx_general;
-        s_maxn = s_maxw = 0;
-        s_flat = 1;
-        s_in_plane = 1;
-    }
     const int2 inactive = make_int2(0, __float_as_int(-1e9f));
     auto act_n = [&](int n) { return len_n[n] >= 0.f; };
     auto act_w = [&](int w) { return win_w[w].y >= 0; };  // the sign bit
-    for (int n = (int)N + tid; n < NP; n += kThreads) {  // padding channels: never active
-        el4[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-        rxp[n] = make_float2(0.f, 0.f);
-        len_n[n] = -1e9f;
-    }
-    for (int w = (int)W + tid; w < WP; w += kThreads) {  // padding waves: zero weight
-        txc[w] = make_float4(0.f, 0.f, 0.f, 0.f);
-        txp[w] = make_float4(0.f, 0.f, 0.f, 0.f);
-        base_w[w] = 0.f;
-        kind_w[w] = USTB_WAVE_ZERO;
-        win_w[w] = inactive;
-    }
-    __syncthreads();  // the shared scalars are set before the loops below change them
     // sub-tile delays [lo, hi] -> window start j after `base` and largest position after
     // that, both in [0, kHalf]; the margin covers the rounding of the bounds
     auto window_part = [&](float base, float lo, float hi, float& j, float& len) {
@@ -453,9 +471,21 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         len = fminf(fmaxf(hi + kMargin - base - j, 0.f), kHalf);
     };
     auto pack_part = [&](float base, float j, float len) { return make_int2((int)base + (int)j, __float_as_int(len)); };
-    auto longest = [&](int& m, float len) { atomicMax(&m, __float_as_int(len)); };
-    for (int64_t n = tid; n < N; n += kThreads) {
-        const float ex = __ldg(A.el + 3 * n), ey = __ldg(A.el + 3 * n + 1), ez = __ldg(A.el + 3 * n + 2);
+    // the largest window position of a warp's channels or waves into m
+    auto longest = [&](int& m, float len) {
+        const int v = __reduce_max_sync(0xffffffffu, __float_as_int(len));
+        if (lane == 0 && v > 0) atomicMax(&m, v);
+    };
+    float longest_n = 0.f, longest_w = 0.f;
+    for (int n = tid; n < NP; n += kThreads) {
+        const float ex = next_el.x, ey = next_el.y, ez = next_el.z;
+        load_el(n + kThreads);
+        if (n >= (int)N) {  // padding channels: never active
+            el4[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+            rxp[n] = make_float2(0.f, 0.f);
+            len_n[n] = -1e9f;
+            continue;
+        }
         float dmin, dmax;
         dist_range(tbox, ex, ey, ez, dmin, dmax);
         float lo = (dmin * A.inv_c + A.lens) * A.fs, hi = (dmax * A.inv_c + A.lens) * A.fs;
@@ -469,17 +499,28 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         float j, len;
         window_part(base, lo, hi, j, len);
         const bool act = rx_active(A, box, ex, ey, ez);
-        if (ez != __ldg(A.el + 2)) s_flat = 0;
+        if (ez != el0_z) s_flat = 0;
         if (A.rx_origin ? ey != A.oy : (box.lo[1] != ey || box.hi[1] != ey)) s_in_plane = 0;
         el4[n] = make_float4(ex, ey, ez, base);
         rxp[n] = make_float2(frac_cycles(fd_fs * (double)base), j);
         len_n[n] = act ? len : -1e9f;
-        if (act) longest(s_maxn, len);
+        if (act) longest_n = fmaxf(longest_n, len);
     }
-    for (int64_t w = tid; w < W; w += kThreads) {
-        const ustb_wave wv = A.waves[w];
-        kind_w[w] = (unsigned char)wv.kind;
-        if (wv.kind == USTB_WAVE_TABLE) continue;  // bases from the table below
+    for (int w = wtid; w < WP; w += kThreads) {
+        const ustb_wave wv = next_wv;
+        load_wave(w + kThreads);
+        if (w >= (int)W) {  // padding waves: zero weight
+            txc[w] = make_float4(0.f, 0.f, 0.f, 0.f);
+            txp[w] = make_float4(0.f, 0.f, 0.f, 0.f);
+            base_w[w] = 0.f;
+            kind_w[w] = USTB_WAVE_ZERO;
+            win_w[w] = inactive;
+            continue;
+        }
+        // a table wave without a table has the constant delay -delay
+        const bool table = wv.kind == USTB_WAVE_TABLE;
+        kind_w[w] = (unsigned char)(table && !A.tx_delay_tab ? USTB_WAVE_ZERO : wv.kind);
+        if (table && A.tx_delay_tab) continue;  // bases from the table below
         float lo, hi;
         tx_tau_range(wv, tbox, lo, hi);
         lo = (lo - A.t0) * A.fs;
@@ -487,9 +528,9 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         const float fbase = floorf(lo) - 1.f;
         const bool ok = (hi - fbase <= kHalf - 2.f) && fabsf(fbase) < 1.0e9f;
         const bool act = A.tx_apo_tab != nullptr || wv.apodization != 0.f;
-        if (!ok && act) atomicOr(A.flags, USTB_FLAG_WINDOW_OVERFLOW);
+        if (!ok && act && !table) atomicOr(A.flags, USTB_FLAG_WINDOW_OVERFLOW);
         if (wv.kind == USTB_WAVE_SPHERICAL && act) s_tx_general = 1;
-        if (wv.kind != USTB_WAVE_SPHERICAL && act) s_tx_sph = 0;
+        if (wv.kind != USTB_WAVE_SPHERICAL && act && !table) s_tx_sph = 0;
         const float bw = fminf(fmaxf(fbase, -1.0e9f), 1.0e9f);
         base_w[w] = bw;
         tx_tau_range(wv, box, lo, hi);
@@ -498,9 +539,9 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         float j, len;
         window_part(bw, lo, hi, j, len);
         win_w[w] = act ? pack_part(bw, j, len) : inactive;
-        if (act) longest(s_maxw, len);
+        if (act) longest_w = fmaxf(longest_w, len);
         // s_tx(p) = (tau(p) - t0) fs - base_w; constant part in double
-        const double fs_c = (double)A.fs / (double)wv.sound_speed;
+        const double fs_c = wv.sound_speed == A.c ? A.fs_c : (double)A.fs / (double)wv.sound_speed;
         const double c0 = -((double)wv.delay + (double)A.t0) * (double)A.fs - (double)bw;
         if (wv.kind == USTB_WAVE_PLANE)
             txc[w] = make_float4((float)(wv.dir[0] * fs_c), (float)(wv.dir[1] * fs_c), (float)(wv.dir[2] * fs_c),
@@ -510,8 +551,10 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         else
             txc[w] = make_float4(0.f, 0.f, 0.f, (float)c0);
         txp[w] = make_float4(frac_cycles(fd_fs * ((double)bw + (double)A.t0 * (double)A.fs)), wv.apodization,
-                             (float)fs_c, j);
+                             table ? 0.f : (float)fs_c, j);
     }
+    longest(s_maxn, longest_n);
+    longest(s_maxw, longest_w);
     if (A.tx_delay_tab) {  // tabulated transmit delays: the tile's actual range
         for (int64_t w = 0; w < W; ++w) {
             const ustb_wave wv = A.waves[w];
@@ -536,30 +579,11 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
                 float j, len;
                 window_part(bw, v[0], -v[1], j, len);
                 win_w[w] = pack_part(bw, j, len);
-                longest(s_maxw, len);
+                atomicMax(&s_maxw, __float_as_int(len));
                 txc[w] = make_float4(0.f, 0.f, 0.f, 0.f);
                 txp[w] = make_float4(frac_cycles(fd_fs * ((double)bw + (double)A.t0 * (double)A.fs)),
                                      wv.apodization, 0.f, j);
             }
-        }
-    } else {
-        for (int64_t w = tid; w < W; w += kThreads) {  // table waves without a table: tau = -delay
-            const ustb_wave wv = A.waves[w];
-            if (wv.kind != USTB_WAVE_TABLE) continue;
-            const float lo = (-wv.delay - A.t0) * A.fs;
-            const float fbase = floorf(lo) - 1.f;
-            const bool act = A.tx_apo_tab != nullptr || wv.apodization != 0.f;
-            const float bw = fminf(fmaxf(fbase, -1.0e9f), 1.0e9f);
-            base_w[w] = bw;
-            kind_w[w] = USTB_WAVE_ZERO;
-            float j, len;
-            window_part(bw, lo, lo, j, len);
-            win_w[w] = act ? pack_part(bw, j, len) : inactive;
-            if (act) longest(s_maxw, len);
-            const double c0 = -((double)wv.delay + (double)A.t0) * (double)A.fs - (double)bw;
-            txc[w] = make_float4(0.f, 0.f, 0.f, (float)c0);
-            txp[w] = make_float4(frac_cycles(fd_fs * ((double)bw + (double)A.t0 * (double)A.fs)), wv.apodization,
-                                 0.f, j);
         }
     }
     __syncthreads();
@@ -602,7 +626,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     auto run = [&](auto stage, const int64_t f0, const int nf) {
     using ST = decltype(stage);
     constexpr int CG = ST::CG, KW = ST::KW, SLOT = ST::SLOT, NS = CG * KW;  // NS slots per stage
-    const float2 ph = A.pix_phase ? __ldg(A.pix_phase + p) : make_float2(1.f, 0.f);
+    const float2 ph = MODE != USTB_DIM_BOTH && A.pix_phase ? __ldg(A.pix_phase + p) : make_float2(1.f, 0.f);
     const float fdfs = (float)fd_fs;
     const int Lc = (int)A.L;             // entries per trace
     const uint32_t slots_s = (uint32_t)__cvta_generic_to_shared(slots);
@@ -883,11 +907,17 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     // copied while a stage is computed.  One barrier per stage: it makes the stage's
     // entries visible to every warp and frees the other buffer (read by the stage
     // before) for the next stage's copies.
-    // half = k >= 0: this CTA takes part k of A.split equal parts of the stages and
-    // adds its partial sum to the (zeroed) output; -1: all of them, plain stores
-    const int parts = half < 0 ? 1 : A.split;
-    const int s_lo = half < 0 ? 0 : (int)((int64_t)nstages * half / parts);
-    const int s_hi = half < 0 ? nstages : (int)((int64_t)nstages * (half + 1) / parts);
+    // part = k >= 0: this CTA takes part k of A.split equal parts of the work; -1: all of it.
+    // dimension.both: of the stages, whose partial sums are added (store_both).  transmit
+    // and receive: of the outer list (channel groups, wave chunks), whose outputs are
+    // disjoint; gaps in the list, inactive and so zero, belong to the part before them.
+    const int parts = part < 0 ? 1 : A.split, me = part < 0 ? 0 : part;
+    constexpr bool kByOuter = MODE != USTB_DIM_BOTH;
+    const int n_split = kByOuter ? no : nstages;
+    const int u_lo = (int)((int64_t)n_split * me / parts), u_hi = (int)((int64_t)n_split * (me + 1) / parts);
+    const int s_lo = kByOuter ? u_lo * ni * nf : u_lo, s_hi = kByOuter ? u_hi * ni * nf : u_hi;
+    const int out_lo = (kByOuter && me > 0) ? (u_lo < no ? olist[u_lo] : (ORDER_A ? NC : NG)) : 0;
+    const int out_hi = (kByOuter && me + 1 < parts) ? (u_hi < no ? olist[u_hi] : (ORDER_A ? NC : NG)) : (ORDER_A ? NC : NG);
     // list positions (outer, inner), frame, first channel and first wave of a stage
     struct Pos { int o, i, f, n0, w0; };
     auto place_outer = [&](Pos& q) { (ORDER_A ? q.w0 : q.n0) = olist[q.o] * (ORDER_A ? KW : CG); };
@@ -925,20 +955,47 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         slot_base = slot0 + (unsigned)(buf * kBufBytes);
     };
     const float2 zero2 = make_float2(0.f, 0.f);
-    // dimension.both: the pixel's sum, plain store or (split tiles) one of the partial sums
+    // dimension.both: the pixel's sum, plain store or (split tiles) one of the partial sums;
+    // without scratch for those they are added into the zeroed image
     auto store_both = [&](int fr) {
-        const float2 y = CPLX ? cmul(Y[fr], ph) : Y[fr];
+        const int tile = s_where[0], sub = s_where[1], part = s_where[2], parts = part < 0 ? 1 : A.split;
+        const int p = __ldg(A.tiles + (int64_t)tile * kTile + sub * kThreads + tid);
         const int64_t f = f0 + fr;
-        if (half < 0) {
-            store_cube(p + A.f_f * f, y);
-        } else if (live && A.cube) {  // partial sums: two give fl(a + b) in either order; three or
-                                      // four are added in completion order (last-bit differences)
-            if constexpr (CPLX) {
-                atomicAdd(&reinterpret_cast<float2*>(A.cube)[p + A.f_f * f].x, y.x);
-                atomicAdd(&reinterpret_cast<float2*>(A.cube)[p + A.f_f * f].y, y.y);
-            } else {
-                atomicAdd(&reinterpret_cast<float*>(A.cube)[p + A.f_f * f], y.x);
+        const int64_t nsub = A.n_tiles * kSub, u = f * nsub + (int64_t)tile * kSub + sub;
+        float2 y = Y[fr];
+        if (part >= 0 && A.partial) {
+            // every part leaves its sum in its slab; the last one to come adds them in order
+            float2* slab = A.partial + u * parts * kThreads + tid;
+            slab[(int64_t)part * kThreads] = y;
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(A.tickets + u, 1u) == (unsigned)(parts - 1);
+            __syncthreads();
+            if (!s_last) return;
+            __threadfence();
+            y = make_float2(0.f, 0.f);
+            for (int k = 0; k < parts; ++k) {
+                const float2 v = __ldcg(slab + (int64_t)k * kThreads);
+                y.x += v.x;
+                y.y += v.y;
             }
+        }
+        if (!in_image(p) || !A.cube) return;
+        if (CPLX && A.pix_phase) y = cmul(y, __ldg(A.pix_phase + p));
+        const int64_t o = p + A.f_f * f;
+        float2* const co = reinterpret_cast<float2*>(A.cube) + o;
+        float* const ro = reinterpret_cast<float*>(A.cube) + o;
+        if (part >= 0 && !A.partial) {  // two sums give fl(a + b) in either order; three or four are
+                                        // added in completion order (last-bit differences)
+            if constexpr (CPLX) {
+                atomicAdd(&co->x, y.x);
+                atomicAdd(&co->y, y.y);
+            } else {
+                atomicAdd(ro, y.x);
+            }
+        } else {
+            if constexpr (CPLX) *co = y;
+            else *ro = y.x;
         }
     };
 
@@ -973,7 +1030,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             if (oc != cur || (FRAMES && cur_pos.f != cur_f)) {
                 if (cur >= 0) finish_chunk();
                 if (oc != cur) {
-                    zero_chunks(cur + 1, oc);
+                    zero_chunks(cur < 0 ? out_lo : cur + 1, oc);
                     setup_tx(w0);
                 }
                 cur = oc;
@@ -1004,7 +1061,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             else units(std::false_type{});
         }
         if (cur >= 0) finish_chunk();
-        zero_chunks(cur + 1, NC);
+        zero_chunks(cur < 0 ? out_lo : cur + 1, out_hi);
         if (MODE == USTB_DIM_BOTH)
             for (int fr = 0; fr < (FRAMES ? nf : 1); ++fr) store_both(fr);
     } else {
@@ -1097,7 +1154,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             if (og != cur || (FRAMES && cur_pos.f != cur_f)) {
                 if (cur >= 0) finish_group();
                 if (og != cur) {
-                    zero_groups(cur + 1, og);
+                    zero_groups(cur < 0 ? out_lo : cur + 1, og);
                     setup_rx(n0);
                     gmask = 0;
 #pragma unroll
@@ -1116,7 +1173,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             else units(n0, w0, std::integral_constant<int, kMasked>{});
         }
         if (cur >= 0) finish_group();
-        zero_groups(cur + 1, NG);
+        zero_groups(cur < 0 ? out_lo : cur + 1, out_hi);
         if constexpr (MODE == USTB_DIM_BOTH)
             for (int fr = 0; fr < (FRAMES ? nf : 1); ++fr) store_both(fr);
         if constexpr (EPI) {
@@ -1135,12 +1192,14 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     };
     auto frames = [&](auto stage) {
         build_lists(stage);
+        wait_for_entries();
         if constexpr (FRAMES && EPI) {  // the epilogue's sums are one frame's
             for (int64_t f = f_first; f < f_first + nfr; ++f) run(stage, f, 1);
         } else {
             run(stage, f_first, FRAMES ? nfr : 1);
         }
     };
+    // (the zero stores of MODE none and the atomics into the image come after this too)
     if constexpr (CPLX) {
         if (narrow) frames(Stage<SHAPE, true, false>{});
         else frames(Stage<SHAPE, true, true>{});
@@ -1152,10 +1211,8 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
 // One launch per request: grid = (tiles x sub-tiles x CTAs per sub-tile, frames).
 template <int MODE, bool CPLX, bool EPI, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 2) das_fast_kernel(const Params A) {
-    zero_slots();
-    const int parts = MODE == USTB_DIM_BOTH ? A.split : 1;
-    const int b = (int)(blockIdx.x / parts), half = parts >= 2 ? (int)(blockIdx.x % parts) : -1;
-    das_tile<MODE, CPLX, EPI, SHAPE>(A, b / kSub, b % kSub, (int64_t)blockIdx.y, half);
+    const int b = (int)(blockIdx.x / A.split), part = A.split >= 2 ? (int)(blockIdx.x % A.split) : -1;
+    das_tile<MODE, CPLX, EPI, SHAPE>(A, b / kSub, b % kSub, (int64_t)blockIdx.y, part);
 }
 
 // Persistent form: two CTAs per SM pull (request, half tile, frames) work items from a
@@ -1174,7 +1231,7 @@ struct BatchParams {
 template <int MODE, bool CPLX, bool EPI, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 2) das_fast_persistent(const __grid_constant__ BatchParams B) {
     __shared__ long long s_item;
-    zero_slots();
+    bool first = true;
     const int64_t total = B.first_item[B.n];
     for (;;) {
         if (threadIdx.x == 0) s_item = (long long)atomicAdd(B.counter, 1ull);
@@ -1189,7 +1246,8 @@ __global__ void __launch_bounds__(kThreads, 2) das_fast_persistent(const __grid_
         const int64_t subs = A.n_tiles * kSub;
         const int64_t f0 = (local / subs) * A.fpi;
         const int b = (int)(local % subs);
-        das_tile<MODE, CPLX, EPI, SHAPE, true>(A, b / kSub, b % kSub, f0, -1, (int)min((int64_t)A.fpi, A.F - f0));
+        das_tile<MODE, CPLX, EPI, SHAPE, true>(A, b / kSub, b % kSub, f0, -1, (int)min((int64_t)A.fpi, A.F - f0), first);
+        first = false;
     }
 }
 
@@ -1197,6 +1255,24 @@ template <int SHAPE>
 size_t smem_bytes(int64_t N, int64_t W) {
     constexpr int CG = Shape<SHAPE>::CG, KW = Shape<SHAPE>::KW;
     return kBuffers + tile_tables<SHAPE>((N + CG - 1) / CG * CG, (W + KW - 1) / KW * KW).total;
+}
+
+// Launch with leave to start while the kernel before it in the stream ends: the CTAs set
+// their tile up (8 to 10 us of dependent loads and long arithmetic) beside the end of the
+// entries pre-pass.  After anything but a kernel the launch is an ordinary one.
+template <typename K, typename P>
+cudaError_t launch_dependent(K* kern, dim3 grid, size_t smem, cudaStream_t s, const P& params) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, params);
 }
 
 template <int MODE, bool CPLX, bool EPI, int SHAPE>
@@ -1210,18 +1286,16 @@ int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
                  (long long)A.N, (long long)A.W, smem, optin);
     auto kern = das_fast_kernel<MODE, CPLX, EPI, SHAPE>;
     USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // dimension.both with few tiles (under 4 per SM): two CTAs per tile, each over half of
-    // its stages, add their partial sums into the zeroed image, so the last wave of
-    // tiles is half as long.  With many tiles the tail is already short.
-    int sms = 0;
-    USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     Params B = A;
-    if (MODE != USTB_DIM_BOTH) B.split = 1;
-    else if (B.split == 0) B.split = (n_tiles * F < 4 * (int64_t)sms) ? 2 : 1;
-    if (B.split >= 2 && B.cube)
+    if (MODE == USTB_DIM_BOTH && B.split >= 2 && B.cube && !B.partial)
         USTB_CUDA(cudaMemsetAsync(B.cube, 0, (size_t)(B.P * F) * (CPLX ? 8 : 4), s));
     dim3 grid((unsigned)(n_tiles * kSub * B.split), (unsigned)F);
-    kern<<<grid, kThreads, smem, s>>>(B);
+    // only the pre-pass is known to leave the outputs and the geometry alone
+    if (B.after_entries) {
+        USTB_CUDA(launch_dependent(kern, grid, smem, s, B));
+    } else {
+        kern<<<grid, kThreads, smem, s>>>(B);
+    }
     USTB_CUDA(cudaGetLastError());
     return USTB_OK;
 }
