@@ -37,10 +37,17 @@ static WinCoeffs window_coeffs(int win) {
 // else the library's choice.  Returns the Shape<> index.
 // dimension.both: 8 x 4 for complex data, 16 x 2 for real data, whose sums take half the
 // registers (complex 16 x 2 spills).
-int shape_for(int dim, bool cplx, int32_t requested) {
+// dimension.receive, waves outer: 4 x 8, 8 x 4 up to eight waves and 16 x 2 for one or
+// two, whose slots would be padding otherwise (2 x 16, on request, leaves most of its
+// slots empty for few waves, and its sums spill).  2 x 16 / 4 x 8 / 8 x 4 / 16 x 2, us,
+// 128 complex channels on 120 x 90 pixels: 2 waves 82 / - / 41 / 37, 4 waves
+// 94 / 58 / 47 / 38, 8 waves 112 / 70 / 50 / 63, 16 waves 133 / 76 / 84 / 88, 75 waves
+// 310 / 237 / 239 / -; 64 real channels on 200 x 200: 4 waves 45 / 31 / 27 / 33, 8 waves
+// 53 / 33 / 31 / 40, 75 waves 156 / 129 / 154 / -.
+int shape_for(int dim, bool cplx, int32_t requested, int64_t W) {
     if (requested > 0) return requested - 1;
     switch (dim) {
-        case USTB_DIM_RECEIVE: return 0;
+        case USTB_DIM_RECEIVE: return W <= 2 ? 4 : W <= 8 ? 3 : 5;
         case USTB_DIM_BOTH: return cplx ? 1 : 2;
         default: return 1;
     }
@@ -67,7 +74,7 @@ int parts_for(const Params& A, int dim, bool epi, int32_t requested, int& parts)
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    constexpr int kCG[3] = {2, 8, 16}, kKW[3] = {16, 4, 2};
+    constexpr int kCG[6] = {2, 8, 16, 8, 16, 4}, kKW[6] = {16, 4, 2, 4, 2, 8};
     const int64_t groups = (A.N + kCG[A.shape] - 1) / kCG[A.shape], chunks = (A.W + kKW[A.shape] - 1) / kKW[A.shape];
     const int64_t most = dim == USTB_DIM_RECEIVE ? chunks : dim == USTB_DIM_TRANSMIT ? groups : groups * chunks;
     const double stages = (double)groups * (double)chunks;
@@ -292,7 +299,7 @@ static int make_params(const void* ch, int32_t storage, int32_t is_complex, int6
                      (dimension == USTB_DIM_RECEIVE) == (g->stage_shape == 1),
                  USTB_E_ARG, "stage_shape %d does not fit dimension %d (receive: 1; transmit/none: 2 or 3)",
                  (int)g->stage_shape, (int)dimension);
-    A.shape = shape_for(dimension, is_complex != 0, g->stage_shape);
+    A.shape = shape_for(dimension, is_complex != 0, g->stage_shape, W);
     A.split = 1;
     const int rc = parts_for(A, dimension, epilogue != 0, g->ctas_per_tile, A.split);
     if (rc) return rc;
@@ -411,7 +418,7 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
             return rc;
         }
         frames[i] = q.F;
-        if (!empty) key[i] = ((q.dimension * 2 + q.is_complex) * 2 + (q.epilogue ? 1 : 0)) * 4 + P[i].shape;
+        if (!empty) key[i] = ((q.dimension * 2 + q.is_complex) * 2 + (q.epilogue ? 1 : 0)) * 8 + P[i].shape;
     }
     // every request's entry array: carved from the caller's workspace, or allocated
     // from the library pool and freed (stream-ordered) after the launches

@@ -264,8 +264,9 @@ __device__ __forceinline__ bool rx_active(const Params& A, const Box& b, float e
 //            the receive geometry is formed once per (pixel, channel) and the
 //            transmit geometry once per stage
 //   shape 2: channels outer (16 channels x 2 waves)
+//   shapes 3, 4, 5: waves outer (8 x 4, 16 x 2, 4 x 8), dimension.receive
 // dimension.receive needs waves outer, dimension.transmit/none channels outer;
-// dimension.both runs with any of the three.  A sub-tile of complex data whose windows
+// dimension.both runs with any of the first three.  A sub-tile of complex data whose windows
 // do not fit 80-entry slots runs half-size stages with 160-entry slots (half the
 // channels of a waves-outer stage, half the waves of a channels-outer one) in the same
 // buffers; real entries are half as large and always have 160-entry slots.
@@ -285,6 +286,21 @@ template <>
 struct Shape<2> {
     static constexpr bool WAVES_OUTER = false;
     static constexpr int CG = 16, KW = 2;
+};
+template <>
+struct Shape<3> {
+    static constexpr bool WAVES_OUTER = true;
+    static constexpr int CG = 8, KW = 4;
+};
+template <>
+struct Shape<4> {
+    static constexpr bool WAVES_OUTER = true;
+    static constexpr int CG = 16, KW = 2;
+};
+template <>
+struct Shape<5> {
+    static constexpr bool WAVES_OUTER = true;
+    static constexpr int CG = 4, KW = 8;
 };
 template <int SHAPE, bool CPLX, bool WIDE>
 struct Stage {
@@ -1353,7 +1369,11 @@ int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t*
         case USTB_DIM_NONE:
             if (shape == 2) USTB_RUN(USTB_DIM_NONE, false, 2);
             USTB_RUN(USTB_DIM_NONE, false, 1);
-        case USTB_DIM_RECEIVE: USTB_RUN(USTB_DIM_RECEIVE, false, 0);
+        case USTB_DIM_RECEIVE:
+            if (shape == 3) USTB_RUN(USTB_DIM_RECEIVE, false, 3);
+            if (shape == 4) USTB_RUN(USTB_DIM_RECEIVE, false, 4);
+            if (shape == 5) USTB_RUN(USTB_DIM_RECEIVE, false, 5);
+            USTB_RUN(USTB_DIM_RECEIVE, false, 0);
         case USTB_DIM_TRANSMIT:
             if constexpr (CPLX)
                 if (epi) {
