@@ -10,8 +10,14 @@ constexpr int kTile = USTB_TILE_PIXELS;
 constexpr int kThreads = 256;  // threads of a beamforming CTA
 constexpr int kSub = 2;        // sub-tiles (CTAs) per tile
 
+// Interpolation entries of a sample: {x_i, x_{i+1} - x_i} in FP32, or for complex 16-bit
+// storage {x_i, x_{i+1}} as they are stored.
+enum EntryKind { kEntReal = 0, kEntComplex = 1, kEntHalf = 2, kEntBf16 = 3 };
+constexpr int entry_size(int ent) { return ent == kEntComplex ? 16 : 8; }
+
 struct Params {
-    const void* entries;  // [F][W][N][Lp] interpolation entries (float4 complex, float2 real)
+    const void* entries;  // [F][W][N][Lp] interpolation entries of kind `ent`
+    int ent;
     int64_t L, Lp, N, W, F, P;
     const float* el;
     const float* px;
@@ -49,7 +55,7 @@ struct Params {
 
 // Kernel variant of (dimension, epilogue, stage shape) for one request kind: one grid
 // launch of reqs[0] (BATCH false) or one persistent launch of n requests.
-template <bool CPLX, bool BATCH>
+template <int ENT, bool BATCH>
 int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t* frames, int n,
                  unsigned long long* counter, int64_t nt, int64_t F, cudaStream_t s, int max_ctas);
 

@@ -46,7 +46,10 @@
 // inner for .transmit and .none (tx weight per unit).
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
 #include "das_fast.cuh"
@@ -209,10 +212,25 @@ __device__ __forceinline__ void block_min(float (&v)[NV], int* red) {
     }
 }
 
-template <bool CPLX>
-struct EntryT { using type = float4; };
+// {x_i, x_{i+1} - x_i} in FP32, or {x_i, x_{i+1}} as stored, whose difference the unit forms
+template <int ENT>
+struct EntryT { using type = uint2; };
 template <>
-struct EntryT<false> { using type = float2; };
+struct EntryT<kEntReal> { using type = float2; };
+template <>
+struct EntryT<kEntComplex> { using type = float4; };
+
+// a stored 16-bit pair in FP32 (exact)
+template <int ENT>
+__device__ __forceinline__ float2 unpack16(unsigned v) {
+    if constexpr (ENT == kEntHalf) {
+        __half2 h;
+        memcpy(&h, &v, 4);
+        return __half22float2(h);
+    } else {
+        return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    }
+}
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -302,12 +320,12 @@ struct Shape<5> {
     static constexpr bool WAVES_OUTER = true;
     static constexpr int CG = 4, KW = 8;
 };
-template <int SHAPE, bool CPLX, bool WIDE>
+template <int SHAPE, bool BIG, bool WIDE>
 struct Stage {
     static constexpr int CG = (WIDE && Shape<SHAPE>::WAVES_OUTER) ? Shape<SHAPE>::CG / 2 : Shape<SHAPE>::CG;
     static constexpr int KW = (WIDE && !Shape<SHAPE>::WAVES_OUTER) ? Shape<SHAPE>::KW / 2 : Shape<SHAPE>::KW;
-    static constexpr int SLOT = (WIDE || !CPLX) ? 160 : 80;  // entries per (channel, wave) window
-    static_assert(CG * KW * SLOT * (CPLX ? 16 : 8) == kBufBytes, "a stage fills one buffer");
+    static constexpr int SLOT = (WIDE || !BIG) ? 160 : 80;  // entries per (channel, wave) window
+    static_assert(CG * KW * SLOT * (BIG ? 16 : 8) == kBufBytes, "a stage fills one buffer");
 };
 
 // Shared memory of one CTA: kRing stage buffers, then the per-tile tables (their size
@@ -371,14 +389,15 @@ __device__ __forceinline__ float frac_cycles(double v) { return (float)(v - floo
 // FRAMES (persistent kernel): frames f_first .. f_first + nfr - 1 of the tile in turn,
 // after one build of the tile's tables and stage lists (the geometry is the same for
 // every frame of a request).
-template <int MODE, bool CPLX, bool EPI, int SHAPE, bool FRAMES = false>
+template <int MODE, int ENT, bool EPI, int SHAPE, bool FRAMES = false>
 __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int64_t f_first, int part = -1,
                                          int nfr = 1, bool first = true) {
     constexpr bool ORDER_A = Shape<SHAPE>::WAVES_OUTER;
     static_assert(MODE != USTB_DIM_RECEIVE || ORDER_A, "dimension.receive keeps waves outer");
     static_assert((MODE != USTB_DIM_TRANSMIT && MODE != USTB_DIM_NONE) || !ORDER_A,
                   "dimension.transmit / none keep channels outer");
-    using Entry = typename EntryT<CPLX>::type;
+    constexpr bool CPLX = ENT != kEntReal, BIG = ENT == kEntComplex;
+    using Entry = typename EntryT<ENT>::type;
     constexpr int ES = (int)sizeof(Entry);
 
     const int64_t N = A.N, W = A.W, P = A.P;
@@ -608,8 +627,8 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     // any unit inside its slot: receive parts in [0, hn], transmit parts in [0, hw],
     // hn + hw + 1 at most the entries per slot.
     const float maxn = __int_as_float(s_maxn), maxw = __int_as_float(s_maxw);
-    constexpr float kNarrowEnd = (float)Stage<SHAPE, CPLX, false>::SLOT - 1.125f;
-    const bool narrow = CPLX && maxn + maxw <= kNarrowEnd;
+    constexpr float kNarrowEnd = (float)Stage<SHAPE, BIG, false>::SLOT - 1.125f;
+    const bool narrow = BIG && maxn + maxw <= kNarrowEnd;
     const float hn = narrow ? maxn : kHalf, hw = narrow ? kNarrowEnd - maxn : kHalf;
 
     // The stages are every (active outer, active inner) pair of channel groups and wave
@@ -709,7 +728,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
                 if ((unsigned)(win_i0 + j) < (unsigned)Lc) {
                     cp_async<ES>(dst + (uint32_t)(j * ES), win_src + j);
                 } else {
-                    if constexpr (CPLX)
+                    if constexpr (BIG)
                         asm volatile("st.shared.v4.f32 [%0], {%1, %1, %1, %1};\n" ::"r"(dst + (uint32_t)(j * ES)), "f"(0.f) : "memory");
                     else
                         asm volatile("st.shared.v2.f32 [%0], {%1, %1};\n" ::"r"(dst + (uint32_t)(j * ES)), "f"(0.f) : "memory");
@@ -883,7 +902,12 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     auto interp = [&](int c, int k, float t, float b) -> float2 {
         const unsigned addr = (unsigned)__float_as_int(t) * (unsigned)sizeof(Entry) + slot_base +
                               (unsigned)((c * KW + k) * SLOT * (int)sizeof(Entry));
-        if constexpr (CPLX) {
+        if constexpr (ENT == kEntHalf || ENT == kEntBf16) {
+            unsigned a, d;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(a), "=r"(d) : "r"(addr));
+            const float2 x = unpack16<ENT>(a), n = unpack16<ENT>(d);
+            return make_float2(fmaf(b, n.x - x.x, x.x), fmaf(b, n.y - x.y, x.y));
+        } else if constexpr (CPLX) {
             float4 e;
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
                          : "=f"(e.x), "=f"(e.y), "=f"(e.z), "=f"(e.w) : "r"(addr));
@@ -1216,7 +1240,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         }
     };
     // (the zero stores of MODE none and the atomics into the image come after this too)
-    if constexpr (CPLX) {
+    if constexpr (BIG) {
         if (narrow) frames(Stage<SHAPE, true, false>{});
         else frames(Stage<SHAPE, true, true>{});
     } else {
@@ -1225,10 +1249,10 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
 }
 
 // One launch per request: grid = (tiles x sub-tiles x CTAs per sub-tile, frames).
-template <int MODE, bool CPLX, bool EPI, int SHAPE>
+template <int MODE, int ENT, bool EPI, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 2) das_fast_kernel(const Params A) {
     const int b = (int)(blockIdx.x / A.split), part = A.split >= 2 ? (int)(blockIdx.x % A.split) : -1;
-    das_tile<MODE, CPLX, EPI, SHAPE>(A, b / kSub, b % kSub, (int64_t)blockIdx.y, part);
+    das_tile<MODE, ENT, EPI, SHAPE>(A, b / kSub, b % kSub, (int64_t)blockIdx.y, part);
 }
 
 // Persistent form: two CTAs per SM pull (request, half tile, frames) work items from a
@@ -1244,7 +1268,7 @@ struct BatchParams {
     unsigned long long* counter;        // queue head (device scratch, zeroed per launch)
 };
 
-template <int MODE, bool CPLX, bool EPI, int SHAPE>
+template <int MODE, int ENT, bool EPI, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 2) das_fast_persistent(const __grid_constant__ BatchParams B) {
     __shared__ long long s_item;
     bool first = true;
@@ -1262,7 +1286,7 @@ __global__ void __launch_bounds__(kThreads, 2) das_fast_persistent(const __grid_
         const int64_t subs = A.n_tiles * kSub;
         const int64_t f0 = (local / subs) * A.fpi;
         const int b = (int)(local % subs);
-        das_tile<MODE, CPLX, EPI, SHAPE, true>(A, b / kSub, b % kSub, f0, -1, (int)min((int64_t)A.fpi, A.F - f0), first);
+        das_tile<MODE, ENT, EPI, SHAPE, true>(A, b / kSub, b % kSub, f0, -1, (int)min((int64_t)A.fpi, A.F - f0), first);
         first = false;
     }
 }
@@ -1291,7 +1315,7 @@ cudaError_t launch_dependent(K* kern, dim3 grid, size_t smem, cudaStream_t s, co
     return cudaLaunchKernelEx(&cfg, kern, params);
 }
 
-template <int MODE, bool CPLX, bool EPI, int SHAPE>
+template <int MODE, int ENT, bool EPI, int SHAPE>
 int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
     const size_t smem = smem_bytes<SHAPE>(A.N, A.W);
     int dev = 0, optin = 0;
@@ -1300,11 +1324,11 @@ int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
     USTB_REQUIRE(smem <= (size_t)optin, USTB_E_SHAPE,
                  "%lld channels / %lld waves need %zu bytes of shared memory per tile (limit %d)",
                  (long long)A.N, (long long)A.W, smem, optin);
-    auto kern = das_fast_kernel<MODE, CPLX, EPI, SHAPE>;
+    auto kern = das_fast_kernel<MODE, ENT, EPI, SHAPE>;
     USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     Params B = A;
     if (MODE == USTB_DIM_BOTH && B.split >= 2 && B.cube && !B.partial)
-        USTB_CUDA(cudaMemsetAsync(B.cube, 0, (size_t)(B.P * F) * (CPLX ? 8 : 4), s));
+        USTB_CUDA(cudaMemsetAsync(B.cube, 0, (size_t)(B.P * F) * (ENT != kEntReal ? 8 : 4), s));
     dim3 grid((unsigned)(n_tiles * kSub * B.split), (unsigned)F);
     // only the pre-pass is known to leave the outputs and the geometry alone
     if (B.after_entries) {
@@ -1316,7 +1340,7 @@ int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
     return USTB_OK;
 }
 
-template <int MODE, bool CPLX, bool EPI, int SHAPE>
+template <int MODE, int ENT, bool EPI, int SHAPE>
 int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long long* counter, int max_ctas,
                  cudaStream_t s) {
     BatchParams B;
@@ -1341,7 +1365,7 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
     if (B.first_item[n] == 0) return USTB_OK;
     USTB_REQUIRE(smem <= (size_t)optin, USTB_E_SHAPE, "a request needs %zu bytes of shared memory per tile (limit %d)",
                  smem, optin);
-    auto kern = das_fast_persistent<MODE, CPLX, EPI, SHAPE>;
+    auto kern = das_fast_persistent<MODE, ENT, EPI, SHAPE>;
     USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     USTB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
     // two CTAs per SM, or fewer (max_ctas pairs) to leave room to launches on other streams
@@ -1354,17 +1378,29 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
 }  // namespace
 
 // Kernel variant of (dimension, epilogue, stage shape) for one request kind.
-template <bool CPLX, bool BATCH>
+template <int ENT, bool BATCH>
 int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t* frames, int n,
              unsigned long long* counter, int64_t nt, int64_t F, cudaStream_t s, int max_ctas) {
     auto run = [&](auto m, auto e, auto sh) {
         constexpr int M = decltype(m)::value, S = decltype(sh)::value;
         constexpr bool E = decltype(e)::value;
-        if constexpr (BATCH) return launch_batch<M, CPLX, E, S>(reqs, frames, n, counter, max_ctas, s);
-        else return launch<M, CPLX, E, S>(reqs[0], nt, F, s);
+        if constexpr (BATCH) return launch_batch<M, ENT, E, S>(reqs, frames, n, counter, max_ctas, s);
+        else return launch<M, ENT, E, S>(reqs[0], nt, F, s);
     };
 #define USTB_RUN(M, E, S) \
     return run(std::integral_constant<int, M>{}, std::integral_constant<bool, E>{}, std::integral_constant<int, S>{})
+    if constexpr (ENT == kEntHalf || ENT == kEntBf16) {  // only the library's own shapes (entries_for)
+        switch (dim) {
+            case USTB_DIM_RECEIVE:
+                if (shape == 3) USTB_RUN(USTB_DIM_RECEIVE, false, 3);
+                if (shape == 4) USTB_RUN(USTB_DIM_RECEIVE, false, 4);
+                USTB_RUN(USTB_DIM_RECEIVE, false, 5);
+            case USTB_DIM_TRANSMIT:
+                if (epi) USTB_RUN(USTB_DIM_TRANSMIT, true, 1);
+                USTB_RUN(USTB_DIM_TRANSMIT, false, 1);
+            default: USTB_RUN(USTB_DIM_BOTH, false, 1);
+        }
+    } else {
     switch (dim) {
         case USTB_DIM_NONE:
             if (shape == 2) USTB_RUN(USTB_DIM_NONE, false, 2);
@@ -1375,7 +1411,7 @@ int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t*
             if (shape == 5) USTB_RUN(USTB_DIM_RECEIVE, false, 5);
             USTB_RUN(USTB_DIM_RECEIVE, false, 0);
         case USTB_DIM_TRANSMIT:
-            if constexpr (CPLX)
+            if constexpr (ENT == kEntComplex)
                 if (epi) {
                     if (shape == 2) USTB_RUN(USTB_DIM_TRANSMIT, true, 2);
                     USTB_RUN(USTB_DIM_TRANSMIT, true, 1);
@@ -1386,6 +1422,7 @@ int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t*
             if (shape == 0) USTB_RUN(USTB_DIM_BOTH, false, 0);
             if (shape == 2) USTB_RUN(USTB_DIM_BOTH, false, 2);
             USTB_RUN(USTB_DIM_BOTH, false, 1);
+    }
     }
 #undef USTB_RUN
 }
