@@ -1,7 +1,8 @@
 // Plain single-precision DAS on precomputed delay/apodization tables — the
 // drop-in for the reference's das_c (+mex/source/das_c.cpp:355-409).
 //
-// One thread per pixel.  For the summing modes each thread keeps FC frame
+// One thread per pixel, or with few pixels four warps of a CTA that share the channels of
+// 32 pixels (in_parts()).  For the summing modes each thread keeps FC frame
 // accumulators in registers and writes every output element exactly once, so
 // the output needs no clearing.  Per unit the arithmetic follows das_c step by
 // step in single precision, with the same roundings where they decide the
@@ -34,6 +35,21 @@ struct TableArgs {
     const float* d_rx;
     void* out;
     int64_t rx_f, w_f, f_f;
+};
+
+// Threads of a CTA that share a pixel's channels (its parts, whole warps) and this thread's
+// pixel and part.  A CTA takes kThreads / PARTS pixels; with parts, threads beyond the last
+// pixel follow it without storing.
+template <int PARTS>
+struct Place {
+    static constexpr int kPixels = kThreads / PARTS;
+    static_assert(kPixels % 32 == 0, "a part is made of whole warps");
+    const int part = PARTS > 1 ? threadIdx.x / kPixels : 0, px = threadIdx.x - part * kPixels;
+    int64_t p = (int64_t)blockIdx.x * kPixels + px;
+    const bool live;
+    __device__ explicit Place(const TableArgs& A) : live(p < A.P) {
+        if (PARTS > 1 && !live) p = A.P - 1;
+    }
 };
 
 template <bool CPLX, int FC>
@@ -290,13 +306,35 @@ __device__ __forceinline__ void unit_sum(const TableArgs& A, const UnitIdx<IDX>&
     }
 }
 
+// The parts' sums, added in order in part 0 (every thread of the CTA calls).
+template <bool CPLX, int FC, int PARTS>
+__device__ __forceinline__ void sum_parts(const Place<PARTS>& q, Acc<CPLX, FC>& acc) {
+    if constexpr (PARTS > 1) {
+        __shared__ float2 sums[FC][kThreads];
+        __syncthreads();
+#pragma unroll
+        for (int f = 0; f < FC; ++f) sums[f][threadIdx.x] = make_float2(acc.re[f], acc.im[f]);
+        __syncthreads();
+        if (q.part != 0) return;
+#pragma unroll
+        for (int k = 1; k < PARTS; ++k)
+#pragma unroll
+            for (int f = 0; f < FC; ++f) {
+                const float2 v = sums[f][k * Place<PARTS>::kPixels + q.px];
+                acc.re[f] += v.x;
+                acc.im[f] += v.y;
+            }
+    }
+}
+
 // Real data: at most 80 registers (6 CTAs of 128 threads per SM), with the carried unit
 // indices; complex data: the phase of every unit needs more registers.
-template <int MODE, bool CPLX, int FC, typename IDX, bool MAGIC>
+template <int MODE, bool CPLX, int FC, typename IDX, bool MAGIC, int PARTS>
 __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(const TableArgs A) {
-    const int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (p >= A.P) return;
-    const int64_t P = A.P;
+    const Place<PARTS> q(A);
+    if (PARTS == 1 && !q.live) return;
+    const int64_t p = q.p, P = A.P;
+    const bool stores = PARTS == 1 || (q.live && q.part == 0);
     constexpr bool PER_WAVE = (MODE == USTB_DIM_RECEIVE || MODE == USTB_DIM_NONE);
     constexpr int NACC = PER_WAVE ? WC : 1;
     Acc<CPLX, FC> acc[NACC];
@@ -316,14 +354,47 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
             // of the apodization column, so that every wave chunk reads the receive tables
             // of those channels only (the others are skipped per unit anyway)
             int nlo = (int)A.N, nhi = -1;
-            for (int n = 0; n < (int)A.N; ++n)
-                if (ld_stream(A.apo_rx + P * n + p) != 0.0f) {
-                    nlo = min(nlo, n);
-                    nhi = n;
+            if constexpr (PARTS == 1) {
+                for (int n = 0; n < (int)A.N; ++n)
+                    if (ld_stream(A.apo_rx + P * n + p) != 0.0f) {
+                        nlo = min(nlo, n);
+                        nhi = n;
+                    }
+                const unsigned live = __activemask();
+                nlo = __reduce_min_sync(live, nlo);
+                nhi = __reduce_max_sync(live, nhi);
+            } else {  // a part scans its share of the column, eight loads in flight
+                const int per = ((int)A.N + PARTS - 1) / PARTS, end = min((q.part + 1) * per, (int)A.N);
+                for (int n0 = q.part * per; n0 < end; n0 += 8) {
+                    float a[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i] = n0 + i < end ? ld_stream(A.apo_rx + P * (n0 + i) + p) : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (a[i] != 0.0f) {
+                            nlo = min(nlo, n0 + i);
+                            nhi = n0 + i;
+                        }
                 }
-            const unsigned live = __activemask();
-            nlo = __reduce_min_sync(live, nlo);
-            nhi = __reduce_max_sync(live, nhi);
+                nlo = __reduce_min_sync(0xffffffffu, nlo);
+                nhi = __reduce_max_sync(0xffffffffu, nhi);
+                __shared__ int lo[kThreads / 32], hi[kThreads / 32];
+                __syncthreads();
+                if ((threadIdx.x & 31) == 0) {
+                    lo[threadIdx.x / 32] = nlo;
+                    hi[threadIdx.x / 32] = nhi;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < kThreads / 32; ++i) {
+                    nlo = min(nlo, lo[i]);
+                    nhi = max(nhi, hi[i]);
+                }
+                // the CTA's channels in equal parts
+                const int cnt = max(nhi - nlo + 1, 0), first = nlo;
+                nlo = first + cnt * q.part / PARTS;
+                nhi = first + cnt * (q.part + 1) / PARTS - 1;
+            }
             for (int64_t w0 = 0; w0 < A.W; w0 += WC) {
                 const int wc = (int)min((int64_t)WC, A.W - w0);
                 load_tx(w0, wc);
@@ -399,11 +470,17 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
                 if (MODE == USTB_DIM_RECEIVE)
 #pragma unroll
                     for (int k = 0; k < WC; ++k)
-                        if (k < wc) store<CPLX, FC>(A, p + A.w_f * (w0 + k), f0, nf, acc[k]);
+                        if (k < wc) {
+                            sum_parts(q, acc[k]);
+                            if (stores) store<CPLX, FC>(A, p + A.w_f * (w0 + k), f0, nf, acc[k]);
+                        }
             }
-            if (MODE == USTB_DIM_BOTH) store<CPLX, FC>(A, p, f0, nf, acc[0]);
-        } else {
-            for (int64_t n = 0; n < A.N; ++n) {
+            if (MODE == USTB_DIM_BOTH) {
+                sum_parts(q, acc[0]);
+                if (stores) store<CPLX, FC>(A, p, f0, nf, acc[0]);
+            }
+        } else if (q.live) {
+            for (int64_t n = q.part; n < A.N; n += PARTS) {
                 const float rxa = __ldg(A.apo_rx + P * n + p);
                 const float rxd = __ldg(A.d_rx + P * n + p);
                 if (MODE == USTB_DIM_TRANSMIT) acc[0].zero();
@@ -435,11 +512,14 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
 // are swapped in chunk_units (delays and weights add and multiply in either order): the
 // channels' values are the chunk's, the wave's the common one.  The next chunk's receive
 // values are loaded a chunk ahead.
-template <int MODE, bool CPLX, int FC, typename IDX, bool MAGIC>
+template <int MODE, bool CPLX, int FC, typename IDX, bool MAGIC, int PARTS>
 __global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs A) {
-    const int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (p >= A.P) return;
-    const int64_t P = A.P;
+    const Place<PARTS> q(A);
+    if (PARTS == 1 && !q.live) return;
+    const int64_t p = q.p, P = A.P;
+    const bool stores = PARTS == 1 || (q.live && q.part == 0);
+    const int first = q.part * WC;
+    constexpr int step = PARTS * WC;  // chunks of channels of this part
     const int N = (int)A.N, W = (int)A.W;
     constexpr bool PER_CHANNEL = (MODE == USTB_DIM_TRANSMIT || MODE == USTB_DIM_NONE);
     Acc<CPLX, FC> acc[PER_CHANNEL ? WC : 1];
@@ -474,29 +554,31 @@ __global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs 
         if (MODE == USTB_DIM_RECEIVE) {
             for (int w = 0; w < W; ++w) {
                 acc[0].zero();
-                for (int n0 = 0; n0 < N; n0 += WC) {
+                for (int n0 = first; n0 < N; n0 += step) {
                     load_rx(n0, rxd, rxa);
                     if (chunk(n0)) units(n0, w, rxd, rxa);
                 }
-                store<CPLX, FC>(A, p + A.w_f * w, f0, nf, acc[0]);
+                sum_parts(q, acc[0]);
+                if (stores) store<CPLX, FC>(A, p + A.w_f * w, f0, nf, acc[0]);
             }
         } else if (MODE == USTB_DIM_BOTH) {
             acc[0].zero();
             float d1[WC], a1[WC];
-            load_rx(0, d1, a1);
-            for (int n0 = 0; n0 < N; n0 += WC) {
+            load_rx(first, d1, a1);
+            for (int n0 = first; n0 < N; n0 += step) {
 #pragma unroll
                 for (int k = 0; k < WC; ++k) {
                     rxd[k] = d1[k];
                     rxa[k] = a1[k];
                 }
-                load_rx(n0 + WC, d1, a1);
+                load_rx(n0 + step, d1, a1);
                 if (!chunk(n0)) continue;
                 for (int w = 0; w < W; ++w) units(n0, w, rxd, rxa);
             }
-            store<CPLX, FC>(A, p, f0, nf, acc[0]);
-        } else {
-            for (int n0 = 0; n0 < N; n0 += WC) {
+            sum_parts(q, acc[0]);
+            if (stores) store<CPLX, FC>(A, p, f0, nf, acc[0]);
+        } else if (q.live) {
+            for (int n0 = first; n0 < N; n0 += step) {
                 load_rx(n0, rxd, rxa);
                 const bool any = chunk(n0);
                 auto put = [&](int64_t o) {
@@ -520,39 +602,76 @@ __global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs 
     }
 }
 
+// Whether the four warps of a CTA share 32 pixels' channels (PARTS 4) instead of taking
+// 128 pixels.  Few pixels leave SMs without a CTA or end in a long last round; with many,
+// the warps of a CTA no longer read neighbouring pixels' sample lines together.  The line
+// lies at the CTAs of 128 pixels per SM; one part / four, us, N channels x W waves:
+//   2000 pixels 64 x 16 x 2 frames, complex: both 147 / 44, receive 76 / 29, transmit 100 / 29
+//   10,000 pixels 128 x 16: complex both 85 / 34, real 73 / 35
+//   80,000 pixels 128 x 16 (4 per SM): complex both 196 / 155, receive 199 / 190, transmit
+//     394 / 309; real 149 / 136, 164 / 162, 273 / 206
+//   160,000 pixels 128 x 16 (8 per SM): complex both 315 / 293, receive 322 / 372, transmit
+//     591 / 569; real 248 / 253, 283 / 311, 476 / 369; 1 wave, transmit, 84 / 83 and 54 / 56
+//   160,000 pixels 128 x 75: complex both 1199 / 1089
+//   40,000 pixels 64 x 16 x 2 frames (2 per SM): complex receive 70 / 75
+//   320,000 pixels 64 x 16: complex both 283 / 314, receive 306 / 442
+// A part needs channels of its own (chunks of WC).
+int in_parts(int mode, bool cplx, const TableArgs& A, bool& parts) {
+    int dev = 0, sms = 0;
+    USTB_CUDA(cudaGetDevice(&dev));
+    USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const bool few = A.W <= few_waves(mode);
+    const int64_t per_sm = mode == USTB_DIM_RECEIVE && !few                                             ? 2
+                           : (mode == USTB_DIM_BOTH && cplx) || (mode == USTB_DIM_TRANSMIT && !few) ? 9
+                                                                                                        : 5;
+    parts = A.N >= 4 * WC && A.P <= per_sm * sms * kThreads;
+    return USTB_OK;
+}
+
 template <int MODE, bool CPLX, typename IDX, bool MAGIC>
-void launch_idx(const TableArgs& A, cudaStream_t s) {
-    const unsigned grid = (unsigned)((A.P + kThreads - 1) / kThreads);
-    auto start = [&](auto fc) {
-        constexpr int FC = decltype(fc)::value;
-        if (A.W <= few_waves(MODE)) das_table_few_waves<MODE, CPLX, FC, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
-        else das_table_kernel<MODE, CPLX, FC, IDX, MAGIC><<<grid, kThreads, 0, s>>>(A);
+int launch_idx(const TableArgs& A, cudaStream_t s) {
+    auto start = [&](auto fc, auto parts) {
+        constexpr int FC = decltype(fc)::value, PARTS = decltype(parts)::value, per = kThreads / PARTS;
+        const unsigned grid = (unsigned)((A.P + per - 1) / per);
+        if (A.W <= few_waves(MODE)) das_table_few_waves<MODE, CPLX, FC, IDX, MAGIC, PARTS><<<grid, kThreads, 0, s>>>(A);
+        else das_table_kernel<MODE, CPLX, FC, IDX, MAGIC, PARTS><<<grid, kThreads, 0, s>>>(A);
     };
-    if (A.F == 1) start(std::integral_constant<int, 1>{});
-    else if (A.F == 2) start(std::integral_constant<int, 2>{});
-    else start(std::integral_constant<int, 4>{});
+    auto frames = [&](auto parts) {
+        if (A.F == 1) start(std::integral_constant<int, 1>{}, parts);
+        else if (A.F == 2) start(std::integral_constant<int, 2>{}, parts);
+        else start(std::integral_constant<int, 4>{}, parts);
+    };
+    if constexpr (sizeof(IDX) == 4 && MAGIC) {  // the others are for data of gigabytes
+        bool parts = false;
+        const int rc = in_parts(MODE, CPLX, A, parts);
+        if (rc) return rc;
+        if (parts) {
+            frames(std::integral_constant<int, 4>{});
+            return USTB_OK;
+        }
+    }
+    frames(std::integral_constant<int, 1>{});
+    return USTB_OK;
 }
 
 // 32-bit sample indices when every index of the call (and one past it) fits 31 bits;
 // the float trick of trunc_floor for traces of at most 2^23 samples
 template <int MODE, bool CPLX>
-void launch_fc(const TableArgs& A, cudaStream_t s) {
+int launch_fc(const TableArgs& A, cudaStream_t s) {
     const bool short_traces = A.L <= ((int64_t)1 << 23);
     if (A.LNW * A.F < (int64_t)INT32_MAX - 1 && short_traces)
-        launch_idx<MODE, CPLX, int32_t, true>(A, s);
-    else if (short_traces)
-        launch_idx<MODE, CPLX, int64_t, true>(A, s);
-    else
-        launch_idx<MODE, CPLX, int64_t, false>(A, s);
+        return launch_idx<MODE, CPLX, int32_t, true>(A, s);
+    if (short_traces) return launch_idx<MODE, CPLX, int64_t, true>(A, s);
+    return launch_idx<MODE, CPLX, int64_t, false>(A, s);
 }
 
 template <bool CPLX>
-void launch_mode(int dim, const TableArgs& A, cudaStream_t s) {
+int launch_mode(int dim, const TableArgs& A, cudaStream_t s) {
     switch (dim) {
-        case USTB_DIM_NONE: launch_fc<USTB_DIM_NONE, CPLX>(A, s); break;
-        case USTB_DIM_RECEIVE: launch_fc<USTB_DIM_RECEIVE, CPLX>(A, s); break;
-        case USTB_DIM_TRANSMIT: launch_fc<USTB_DIM_TRANSMIT, CPLX>(A, s); break;
-        default: launch_fc<USTB_DIM_BOTH, CPLX>(A, s); break;
+        case USTB_DIM_NONE: return launch_fc<USTB_DIM_NONE, CPLX>(A, s);
+        case USTB_DIM_RECEIVE: return launch_fc<USTB_DIM_RECEIVE, CPLX>(A, s);
+        case USTB_DIM_TRANSMIT: return launch_fc<USTB_DIM_TRANSMIT, CPLX>(A, s);
+        default: return launch_fc<USTB_DIM_BOTH, CPLX>(A, s);
     }
 }
 
@@ -662,10 +781,8 @@ extern "C" int ustb_das_table_f32(const void* ch, int32_t ch_complex, int64_t L,
     A.out = out;
     const OutStrides os = out_strides(dimension, P, N, W);
     A.rx_f = os.rx_f; A.w_f = os.w_f; A.f_f = os.f_f;
-    if (ch_complex)
-        launch_mode<true>(dimension, A, s);
-    else
-        launch_mode<false>(dimension, A, s);
+    rc = ch_complex ? launch_mode<true>(dimension, A, s) : launch_mode<false>(dimension, A, s);
+    if (rc) return rc;
     USTB_CUDA(cudaGetLastError());
     return USTB_OK;
 }
