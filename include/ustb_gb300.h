@@ -202,12 +202,10 @@ typedef struct {
     float rx_origin[3];
     float cf_threshold;          /* coherence factor: elements with rx apodization > this count in M */
     int32_t ctas_per_tile;       /* dimension.both, one launch per request: 1 to 4 CTAs per half tile,
-                                    each over an equal part of its stages; their sums are added in
-                                    order (ustb_das_fast) or into the image (ustb_das_fast_entries:
-                                    with 3 or 4 in completion order, so repeated runs may differ in
-                                    the last bits).  0 = the library picks from the numbers of tiles
-                                    and stages, up to 8 (2 with ustb_das_fast_entries); transmit and
-                                    receive split the same way and ignore this */
+                                    each over an equal part of its stages; the last to finish adds
+                                    their sums in order, so repeated runs give the same bits.  0 = the
+                                    library picks from the numbers of tiles and stages, up to 8;
+                                    transmit and receive split the same way and ignore this */
     int32_t stage_shape;         /* (channel, wave) pairs per shared-memory stage and loop order:
                                     1 = waves outer, 2 channels x 16 waves (dimension.both / receive);
                                     2 = channels outer, 8 x 4; 3 = channels outer, 16 x 2

@@ -55,35 +55,39 @@ int shape_for(int dim, bool cplx, int32_t requested, int64_t W) {
 
 // CTAs (parts) per sub-tile of a grid launch.  Few sub-tiles leave SMs without work or a
 // last round of long CTAs; each part sets the tile up again.  The number taken minimises
-//   (rounds + 1/4) (set-up + stages / parts),
-// rounds of CTAs (two per SM; half a round at least: one CTA per SM) with a quarter for
-// the uneven end, times a CTA's length in stages (its set-up is worth 2 and one for every
-// 128 channels and waves); another part must shorten it by 1.5 %.  Measured, one part
-// against this rule: synthetic aperture of real traces, 128 x 128, 0.640 and 0.591 ms,
-// 115 x 115 on 223 x 73 pixels, 480 and 225 us; a transmit image of 145 channels x 9 waves
-// on 73 x 252 pixels, 97 and 60 us; 75-wave IQ compounding, 525 us either way.
-// transmit and receive split where their outputs do not overlap (the epilogue sums over
-// channels, so it does not split).
+//   (rounds + uneven) (set-up + stages / parts),
+// rounds of CTAs (two per SM; half a round at least: one CTA per SM) and half a round for
+// CTAs of different lengths, a quarter from one and a half rounds on, times a CTA's length
+// in stages (its set-up is worth 4.5 and one for every 128 channels and waves); another
+// part must shorten it by 1 %, and a part of dimension.both keeps four stages (a call of a
+// few stages is bound by the host).  Measured, one part against this rule: synthetic
+// aperture of real traces, 128 x 128, 640 and 591 us, 115 x 115 on 223 x 73 pixels, 480 and
+// 225; a transmit image of 145 channels x 9 waves on 73 x 252 pixels, 97 and 60; 75-wave IQ
+// compounding, 525 either way.
+// transmit and receive split where their outputs do not overlap; the epilogue's sums over
+// channels are added like dimension.both's (81 channels x 29 waves into 68 x 89 pixels with
+// coherence factors: one part 159 us, three 78).
 int parts_for(const Params& A, int dim, bool epi, int32_t requested, int& parts) {
     parts = 1;
     if (dim == USTB_DIM_BOTH && requested > 0) {
         parts = requested;
         return USTB_OK;
     }
-    if (dim == USTB_DIM_NONE || epi) return USTB_OK;
+    if (dim == USTB_DIM_NONE) return USTB_OK;
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     constexpr int kCG[6] = {2, 8, 16, 8, 16, 4}, kKW[6] = {16, 4, 2, 4, 2, 8};
     const int64_t groups = (A.N + kCG[A.shape] - 1) / kCG[A.shape], chunks = (A.W + kKW[A.shape] - 1) / kKW[A.shape];
-    const int64_t most = dim == USTB_DIM_RECEIVE ? chunks : dim == USTB_DIM_TRANSMIT ? groups : groups * chunks;
+    const int64_t most = dim == USTB_DIM_RECEIVE ? chunks : dim == USTB_DIM_TRANSMIT ? groups : groups * chunks / 4;
     const double stages = (double)groups * (double)chunks;
-    const double setup = 2.0 + (double)(A.N + A.W) / 128.0;  // of a CTA, in stages
+    const double setup = 4.5 + (double)(A.N + A.W) / 128.0;  // of a CTA, in stages
     const double rounds = (double)A.n_tiles * ustb::kSub * (double)A.F / (2.0 * sms);  // of one part each
     double best = 0.0;
     for (int k = 1; k <= 8 && k <= most; ++k) {
-        const double cost = (std::max(k * rounds, 0.5) + 0.25) * (setup + stages / k);
-        if (k == 1 || cost < 0.985 * best) {
+        const double r = std::max(k * rounds, 0.5), uneven = 0.25 + 0.5 * std::min(std::max(1.5 - r, 0.0), 0.5);
+        const double cost = (r + uneven) * (setup + stages / k);
+        if (k == 1 || cost < 0.99 * best) {
             parts = k;
             best = cost;
         }
@@ -105,13 +109,21 @@ __device__ __forceinline__ float2 load_sample(const void* ch, int64_t i) {
     }
 }
 
+// Both entry kernels also zero the tickets of the parts (das_fast.cuh) of the launch that
+// follows them: a memset of its own costs the host as much as a launch.
+__device__ __forceinline__ void zero_tickets(unsigned* tickets, int64_t n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        tickets[i] = 0u;
+}
+
 // Interpolation entries of every trace: E[t][i] = {x_i, x_{i+1} - x_i} for
 // 0 < i < L-1 (das_c.cpp:381-383's validity rule), zero elsewhere.  HBM-bound:
 // one pass over the channel data.
 template <int ST, bool CPLX>
 __global__ void __launch_bounds__(256) build_entries_kernel(const void* __restrict__ ch,
                                                             void* __restrict__ entries, int64_t L, int64_t Lp,
-                                                            int64_t n_traces) {
+                                                            int64_t n_traces, unsigned* tickets, int64_t n_tickets) {
+    zero_tickets(tickets, n_tickets);
     // CTAs stride over traces, threads over the samples of a trace (no 64-bit divisions)
     for (int64_t t = blockIdx.x; t < n_traces; t += gridDim.x) {
         const int64_t in0 = t * L, out0 = t * Lp;
@@ -130,7 +142,9 @@ __global__ void __launch_bounds__(256) build_entries_kernel(const void* __restri
 
 // The same for complex 16-bit samples as they are stored: E[t][i] = {x_i, x_{i+1}}.
 __global__ void __launch_bounds__(256) build_pairs_kernel(const unsigned* __restrict__ ch, uint2* __restrict__ entries,
-                                                          int64_t L, int64_t n_traces) {
+                                                          int64_t L, int64_t n_traces, unsigned* tickets,
+                                                          int64_t n_tickets) {
+    zero_tickets(tickets, n_tickets);
     for (int64_t t = blockIdx.x; t < n_traces; t += gridDim.x) {
         const unsigned* x = ch + t * L;
         uint2* e = entries + t * L;
@@ -181,9 +195,10 @@ cudaMemPool_t entry_pool(int dev) {
     return pools[dev];
 }
 
-// Fill one request's entry array `dst` (entry_bytes(...) bytes of device memory).
+// Fill one request's entry array `dst` (entry_bytes(...) bytes of device memory) and zero
+// its tickets.
 int fill_entries(const void* ch, int32_t storage, int ent, int64_t L, int64_t N, int64_t W, int64_t F, void* dst,
-                 cudaStream_t s) {
+                 cudaStream_t s, unsigned* tickets = nullptr, int64_t n_tickets = 0) {
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -191,45 +206,59 @@ int fill_entries(const void* ch, int32_t storage, int ent, int64_t L, int64_t N,
     if (total == 0) return USTB_OK;
     const unsigned grid = (unsigned)std::min<int64_t>(traces, (int64_t)sms * 32);
     if (ent == ustb::kEntHalf || ent == ustb::kEntBf16) {
-        build_pairs_kernel<<<grid, 256, 0, s>>>(static_cast<const unsigned*>(ch), static_cast<uint2*>(dst), L, traces);
+        build_pairs_kernel<<<grid, 256, 0, s>>>(static_cast<const unsigned*>(ch), static_cast<uint2*>(dst), L, traces,
+                                                tickets, n_tickets);
         USTB_CUDA(cudaGetLastError());
         return USTB_OK;
     }
     switch (storage * 2 + (ent == ustb::kEntComplex ? 1 : 0)) {
-        case USTB_STORE_F32 * 2 + 1: build_entries_kernel<USTB_STORE_F32, true><<<grid, 256, 0, s>>>(ch, dst, L, L, traces); break;
-        case USTB_STORE_F16 * 2 + 1: build_entries_kernel<USTB_STORE_F16, true><<<grid, 256, 0, s>>>(ch, dst, L, L, traces); break;
-        case USTB_STORE_BF16 * 2 + 1: build_entries_kernel<USTB_STORE_BF16, true><<<grid, 256, 0, s>>>(ch, dst, L, L, traces); break;
-        case USTB_STORE_F32 * 2: build_entries_kernel<USTB_STORE_F32, false><<<grid, 256, 0, s>>>(ch, dst, L, L, traces); break;
-        case USTB_STORE_F16 * 2: build_entries_kernel<USTB_STORE_F16, false><<<grid, 256, 0, s>>>(ch, dst, L, L, traces); break;
-        default: build_entries_kernel<USTB_STORE_BF16, false><<<grid, 256, 0, s>>>(ch, dst, L, L, traces); break;
+        case USTB_STORE_F32 * 2 + 1: build_entries_kernel<USTB_STORE_F32, true><<<grid, 256, 0, s>>>(ch, dst, L, L, traces, tickets, n_tickets); break;
+        case USTB_STORE_F16 * 2 + 1: build_entries_kernel<USTB_STORE_F16, true><<<grid, 256, 0, s>>>(ch, dst, L, L, traces, tickets, n_tickets); break;
+        case USTB_STORE_BF16 * 2 + 1: build_entries_kernel<USTB_STORE_BF16, true><<<grid, 256, 0, s>>>(ch, dst, L, L, traces, tickets, n_tickets); break;
+        case USTB_STORE_F32 * 2: build_entries_kernel<USTB_STORE_F32, false><<<grid, 256, 0, s>>>(ch, dst, L, L, traces, tickets, n_tickets); break;
+        case USTB_STORE_F16 * 2: build_entries_kernel<USTB_STORE_F16, false><<<grid, 256, 0, s>>>(ch, dst, L, L, traces, tickets, n_tickets); break;
+        default: build_entries_kernel<USTB_STORE_BF16, false><<<grid, 256, 0, s>>>(ch, dst, L, L, traces, tickets, n_tickets); break;
     }
     USTB_CUDA(cudaGetLastError());
     return USTB_OK;
 }
 
-// Allocate (stream-ordered, from the library pool) and fill one request's entries.  Behind
-// them (on a 256-byte boundary) lie ``sums`` bytes and ``tickets`` zeroed bytes; *behind
-// points there.
-int build_entries(const void* ch, int32_t storage, int ent_kind, int64_t L, int64_t N, int64_t W, int64_t F,
-                  void** out, cudaStream_t s, int64_t sums = 0, int64_t tickets = 0, char** behind = nullptr) {
+// Bytes of device memory from the library pool (stream-ordered).
+int pool_alloc(int64_t bytes, const char* what, void** out, cudaStream_t s) {
     *out = nullptr;
-    const int64_t ent = (entry_bytes(L, N, W, F, ent_kind) + 255) & ~int64_t(255), bytes = ent + sums + tickets;
     if (bytes == 0) return USTB_OK;
     int dev = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     cudaMemPool_t pool = entry_pool(dev);
     USTB_REQUIRE(pool, USTB_E_CUDA, "could not create the entry memory pool on device %d", dev);
-    cudaError_t e = cudaMallocFromPoolAsync(out, (size_t)bytes, pool, s);
+    const cudaError_t e = cudaMallocFromPoolAsync(out, (size_t)bytes, pool, s);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         *out = nullptr;
-        ustb::set_error("%lld bytes of interpolation entries: %s", (long long)bytes, cudaGetErrorString(e));
+        ustb::set_error("%lld bytes of %s: %s", (long long)bytes, what, cudaGetErrorString(e));
         return USTB_E_OOM;
     }
-    if (behind) *behind = static_cast<char*>(*out) + ent;
-    // before the entries, so that the beamforming launch follows their kernel
-    if (tickets) USTB_CUDA(cudaMemsetAsync(static_cast<char*>(*out) + ent + sums, 0, (size_t)tickets, s));
+    return USTB_OK;
+}
+
+// Allocate and fill one request's entries.
+int build_entries(const void* ch, int32_t storage, int ent_kind, int64_t L, int64_t N, int64_t W, int64_t F,
+                  void** out, cudaStream_t s) {
+    const int rc = pool_alloc(entry_bytes(L, N, W, F, ent_kind), "interpolation entries", out, s);
+    if (rc || !*out) return rc;
     return fill_entries(ch, storage, ent_kind, L, N, W, F, *out, s);
+}
+
+// Bytes of the sums of a request's parts, where parts are added, and its number of tickets.
+int64_t part_bytes(const Params& A, int dim, bool epi, int64_t& tickets) {
+    tickets = 0;
+    if (A.split <= 1 || (dim != USTB_DIM_BOTH && !epi)) return 0;
+    tickets = A.n_tiles * ustb::kSub * A.F;
+    return tickets * A.split * ustb::kThreads * (epi ? 3 : 1) * (int64_t)sizeof(float2);
+}
+void set_parts(Params& A, void* scratch, int64_t sums) {
+    A.partial = static_cast<float2*>(scratch);
+    A.tickets = reinterpret_cast<unsigned*>(static_cast<char*>(scratch) + sums);
 }
 
 // The launch of reqs' entry kind.
@@ -367,33 +396,24 @@ extern "C" int ustb_das_fast(const void* ch, int32_t storage, int32_t is_complex
     bool empty = false;
     int rc = make_params(ch, storage, is_complex, L, N, W, F, g, dimension, epilogue, out, flags, s, A, empty);
     if (rc || empty) return rc;
-    // partial sums of split sub-tiles and their tickets behind the entries
-    const int64_t nt = g->n_tiles, nsub = nt * ustb::kSub * F;
-    int64_t sums = 0, tickets = 0;
-    if (dimension == USTB_DIM_BOTH && A.split > 1) {
-        sums = nsub * A.split * ustb::kThreads * (int64_t)sizeof(float2);
-        tickets = nsub * (int64_t)sizeof(unsigned);
-    }
+    // entries, then the parts' sums and tickets
+    const int64_t ent_bytes = (entry_bytes(L, N, W, F, A.ent) + 255) & ~int64_t(255);
+    int64_t tickets = 0;
+    const int64_t sums = part_bytes(A, dimension, epilogue != 0, tickets);
     void* ent = nullptr;
-    char* behind = nullptr;
-    rc = build_entries(ch, storage, A.ent, L, N, W, F, &ent, s, sums, tickets, &behind);
-    if (rc == USTB_E_OOM && tickets) {  // room for the entries alone: whole sub-tiles, or sums in the image
+    rc = pool_alloc(ent_bytes + sums + tickets * (int64_t)sizeof(unsigned), "interpolation entries", &ent, s);
+    if (rc == USTB_E_OOM && tickets) {  // room for the entries alone: whole sub-tiles
+        A.split = 1;
         tickets = 0;
-        if (g->ctas_per_tile == 0) A.split = 1;
         ustb::clear_error();
-        rc = build_entries(ch, storage, A.ent, L, N, W, F, &ent, s);
+        rc = pool_alloc(ent_bytes, "interpolation entries", &ent, s);
     }
-    if (rc) {
-        if (ent) (void)cudaFreeAsync(ent, s);
-        return rc;
-    }
+    if (rc) return rc;
     A.entries = ent;
     A.after_entries = true;
-    if (tickets) {
-        A.partial = reinterpret_cast<float2*>(behind);
-        A.tickets = reinterpret_cast<unsigned*>(behind + sums);
-    }
-    rc = dispatch<false>(dimension, epilogue, &A, nullptr, 1, nullptr, nt, F, s, 0);
+    if (tickets) set_parts(A, static_cast<char*>(ent) + ent_bytes, sums);
+    rc = fill_entries(ch, storage, A.ent, L, N, W, F, ent, s, A.tickets, tickets);
+    if (!rc) rc = dispatch<false>(dimension, epilogue, &A, nullptr, 1, nullptr, g->n_tiles, F, s, 0);
     const cudaError_t fe = cudaFreeAsync(ent, s);
     if (rc) return rc;
     USTB_CUDA(fe);
@@ -432,11 +452,25 @@ extern "C" int ustb_das_fast_entries(const void* entries, int32_t is_complex, in
     if (rc || empty) return rc;
     USTB_REQUIRE(((uintptr_t)entries & 15) == 0, USTB_E_ARG, "entries must be 16-byte aligned");
     A.entries = entries;
-    // no scratch here: the parts of dimension.both add into the image, at most two unless
-    // asked for (two sums are the same in either order)
-    if (dimension == USTB_DIM_BOTH && g->ctas_per_tile == 0) A.split = std::min(A.split, 2);
-    const int64_t nt = g->n_tiles;
-    return dispatch<false>(dimension, epilogue, &A, nullptr, 1, nullptr, nt, F, s, 0);
+    int64_t tickets = 0;
+    const int64_t sums = part_bytes(A, dimension, epilogue != 0, tickets);
+    if (!tickets) return dispatch<false>(dimension, epilogue, &A, nullptr, 1, nullptr, g->n_tiles, F, s, 0);
+    void* scratch = nullptr;
+    rc = pool_alloc(sums + tickets * (int64_t)sizeof(unsigned), "partial sums", &scratch, s);
+    if (rc == USTB_E_OOM) {  // whole sub-tiles
+        A.split = 1;
+        ustb::clear_error();
+        return dispatch<false>(dimension, epilogue, &A, nullptr, 1, nullptr, g->n_tiles, F, s, 0);
+    }
+    if (rc) return rc;
+    set_parts(A, scratch, sums);
+    const cudaError_t me = cudaMemsetAsync(A.tickets, 0, (size_t)tickets * sizeof(unsigned), s);
+    if (me == cudaSuccess) rc = dispatch<false>(dimension, epilogue, &A, nullptr, 1, nullptr, g->n_tiles, F, s, 0);
+    const cudaError_t fe = cudaFreeAsync(scratch, s);
+    if (rc) return rc;
+    USTB_CUDA(me);
+    USTB_CUDA(fe);
+    return USTB_OK;
 }
 
 static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t* scratch, void* workspace,

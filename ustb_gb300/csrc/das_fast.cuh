@@ -47,7 +47,7 @@ struct Params {
     uint32_t* flags;
     bool after_entries; // grid kernel: the entries pre-pass is the launch before it
     int split;          // grid kernel: CTAs (parts) per sub-tile
-    float2* partial;    // dimension.both: sums of the parts [F * sub-tiles][split][kThreads], or null
+    float2* partial;    // sums of the parts [F * sub-tiles][split][1, or 3 for the epilogue][kThreads]
     unsigned* tickets;  // parts that have finished, per frame and sub-tile (zeroed)
     int shape;  // stage shape (Shape<> index)
     int fpi;    // persistent kernel: frames per work item (one tile, consecutive frames)

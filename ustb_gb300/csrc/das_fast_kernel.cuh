@@ -995,48 +995,44 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         slot_base = slot0 + (unsigned)(buf * kBufBytes);
     };
     const float2 zero2 = make_float2(0.f, 0.f);
-    // dimension.both: the pixel's sum, plain store or (split tiles) one of the partial sums;
-    // without scratch for those they are added into the zeroed image
+    // Every part of a sub-tile leaves its sums in its slab; the last one to come (true)
+    // adds them in order.
+    auto sum_of_parts = [&](auto& v, int tile, int sub, int part, int64_t f) {
+        constexpr int NV = (int)(sizeof(v) / sizeof(v[0]));
+        const int parts = A.split;
+        const int64_t u = f * A.n_tiles * kSub + (int64_t)tile * kSub + sub;
+        float2* slab = A.partial + u * parts * NV * kThreads + tid;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) slab[(int64_t)(part * NV + i) * kThreads] = v[i];
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(A.tickets + u, 1u) == (unsigned)(parts - 1);
+        __syncthreads();
+        if (!s_last) return false;
+        __threadfence();
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = make_float2(0.f, 0.f);
+        for (int k = 0; k < parts; ++k)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const float2 a = __ldcg(slab + (int64_t)(k * NV + i) * kThreads);
+                v[i].x += a.x;
+                v[i].y += a.y;
+            }
+        return true;
+    };
+    // dimension.both: the pixel's sum (of all parts)
     auto store_both = [&](int fr) {
-        const int tile = s_where[0], sub = s_where[1], part = s_where[2], parts = part < 0 ? 1 : A.split;
+        const int tile = s_where[0], sub = s_where[1], part = s_where[2];
         const int p = __ldg(A.tiles + (int64_t)tile * kTile + sub * kThreads + tid);
         const int64_t f = f0 + fr;
-        const int64_t nsub = A.n_tiles * kSub, u = f * nsub + (int64_t)tile * kSub + sub;
-        float2 y = Y[fr];
-        if (part >= 0 && A.partial) {
-            // every part leaves its sum in its slab; the last one to come adds them in order
-            float2* slab = A.partial + u * parts * kThreads + tid;
-            slab[(int64_t)part * kThreads] = y;
-            __threadfence();
-            __syncthreads();
-            if (tid == 0) s_last = atomicAdd(A.tickets + u, 1u) == (unsigned)(parts - 1);
-            __syncthreads();
-            if (!s_last) return;
-            __threadfence();
-            y = make_float2(0.f, 0.f);
-            for (int k = 0; k < parts; ++k) {
-                const float2 v = __ldcg(slab + (int64_t)k * kThreads);
-                y.x += v.x;
-                y.y += v.y;
-            }
-        }
+        float2 y[1] = {Y[fr]};
+        if (part >= 0 && !sum_of_parts(y, tile, sub, part, f)) return;
         if (!in_image(p) || !A.cube) return;
-        if (CPLX && A.pix_phase) y = cmul(y, __ldg(A.pix_phase + p));
+        if (CPLX && A.pix_phase) y[0] = cmul(y[0], __ldg(A.pix_phase + p));
         const int64_t o = p + A.f_f * f;
-        float2* const co = reinterpret_cast<float2*>(A.cube) + o;
-        float* const ro = reinterpret_cast<float*>(A.cube) + o;
-        if (part >= 0 && !A.partial) {  // two sums give fl(a + b) in either order; three or four are
-                                        // added in completion order (last-bit differences)
-            if constexpr (CPLX) {
-                atomicAdd(&co->x, y.x);
-                atomicAdd(&co->y, y.y);
-            } else {
-                atomicAdd(ro, y.x);
-            }
-        } else {
-            if constexpr (CPLX) *co = y;
-            else *ro = y.x;
-        }
+        if constexpr (CPLX) reinterpret_cast<float2*>(A.cube)[o] = y[0];
+        else reinterpret_cast<float*>(A.cube)[o] = y[0].x;
     };
 
     if constexpr (ORDER_A) {
@@ -1217,7 +1213,17 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         if constexpr (MODE == USTB_DIM_BOTH)
             for (int fr = 0; fr < (FRAMES ? nf : 1); ++fr) store_both(fr);
         if constexpr (EPI) {
-            if (live) {
+            bool whole = true;  // this CTA has the sums over every channel
+            if (!FRAMES && A.split > 1) {
+                float2 v[3] = {eS, make_float2(eI, eM), make_float2(eR, eQ)};
+                whole = sum_of_parts(v, s_where[0], s_where[1], s_where[2], f0);
+                eS = v[0];
+                eI = v[1].x;
+                eM = v[1].y;
+                eR = v[2].x;
+                eQ = v[2].y;
+            }
+            if (live && whole) {
                 const int64_t o = p + P * f0;
                 float cf = (eS.x * eS.x + eS.y * eS.y) / eI * (1.f / eM);
                 if (cf != cf) cf = 0.f;  // NaN -> 0 (coherence_factor.m:132)
@@ -1239,7 +1245,6 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             run(stage, f_first, FRAMES ? nfr : 1);
         }
     };
-    // (the zero stores of MODE none and the atomics into the image come after this too)
     if constexpr (BIG) {
         if (narrow) frames(Stage<SHAPE, true, false>{});
         else frames(Stage<SHAPE, true, true>{});
@@ -1326,15 +1331,12 @@ int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
                  (long long)A.N, (long long)A.W, smem, optin);
     auto kern = das_fast_kernel<MODE, ENT, EPI, SHAPE>;
     USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    Params B = A;
-    if (MODE == USTB_DIM_BOTH && B.split >= 2 && B.cube && !B.partial)
-        USTB_CUDA(cudaMemsetAsync(B.cube, 0, (size_t)(B.P * F) * (ENT != kEntReal ? 8 : 4), s));
-    dim3 grid((unsigned)(n_tiles * kSub * B.split), (unsigned)F);
+    dim3 grid((unsigned)(n_tiles * kSub * A.split), (unsigned)F);
     // only the pre-pass is known to leave the outputs and the geometry alone
-    if (B.after_entries) {
-        USTB_CUDA(launch_dependent(kern, grid, smem, s, B));
+    if (A.after_entries) {
+        USTB_CUDA(launch_dependent(kern, grid, smem, s, A));
     } else {
-        kern<<<grid, kThreads, smem, s>>>(B);
+        kern<<<grid, kThreads, smem, s>>>(A);
     }
     USTB_CUDA(cudaGetLastError());
     return USTB_OK;
