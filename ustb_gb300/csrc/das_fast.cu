@@ -162,14 +162,18 @@ int64_t entry_bytes(int64_t L, int64_t N, int64_t W, int64_t F, int ent) {
 
 // What a request's entries hold.  Complex 16-bit samples keep their storage type: a unit
 // loads 8 bytes of shared memory instead of 16 and forms the difference itself, in the
-// same FP32 roundings, and the pre-pass writes half as much.  Measured, FP32
-// entries against these: sector of 256 x 512 pixels with coherence factors 295 and 285 us,
-// matrix volume 7.73 and 7.64 ms, int16 ensemble of 50 frames 4.63 and 4.50 ms.
-// Kept to the shapes that the library picks and to summed images (dimension.none is bound
-// by its stores).
+// same FP32 roundings, and the pre-pass writes half as much.  Measured, FP32 entries
+// against these: matrix volume 7.74 and 7.22 ms, int16 ensemble of 50 frames 4.62 and 4.14
+// ms, sector with coherence factors 300 and 272 us; 200 x 200 pixels x 4 frames, 32 waves,
+// 424 and 345 us (its windows need the half-size stages with FP32 entries), 400 x 400
+// pixels, 75 waves, 517 and 507 us.  FP32 entries stay for one or two waves (7 draws of
+// them 0 to 12 % slower here), receive images of more than eight waves (50 waves on
+// 297 x 455 pixels 297 and 323 us), dimension.none (bound by its stores) and the shapes
+// that are asked for.
 int entries_for(int32_t storage, bool cplx, int dim, int shape, int64_t W) {
     if (!cplx) return ustb::kEntReal;
-    if (storage == USTB_STORE_F32 || dim == USTB_DIM_NONE || shape != shape_for(dim, true, 0, W))
+    if (storage == USTB_STORE_F32 || dim == USTB_DIM_NONE || W <= 2 || (dim == USTB_DIM_RECEIVE && W > 8) ||
+        shape != shape_for(dim, true, 0, W))
         return ustb::kEntComplex;
     return storage == USTB_STORE_F16 ? ustb::kEntHalf : ustb::kEntBf16;
 }
