@@ -148,7 +148,7 @@ __device__ __forceinline__ void prefetch_units(const TableArgs& A, IDX nL, const
 template <bool CPLX, int FC, bool PER_WAVE, int NACC, typename IDX, bool MAGIC, bool PACK>
 __device__ __forceinline__ void chunk_units(const TableArgs& A, IDX nL, const IDX* wbase, int wc, int64_t f0,
                                             int nf, const float* txd, const float* txa, float rxd, float rxa,
-                                            Acc<CPLX, FC>* acc, bool pf = false, int dn = 0) {
+                                            Acc<CPLX, FC>* acc, bool pf = false, int dn = 0, IDX ahead = 0) {
     float a[WC], b[WC], wr[WC], wi[WC];
     IDX base[WC];
     bool ok[WC];
@@ -158,7 +158,7 @@ __device__ __forceinline__ void chunk_units(const TableArgs& A, IDX nL, const ID
         if (pf && k < wc) {
             const int m = min(max(n0 + dn, 1), Lm1 - 1);
             const char* x = reinterpret_cast<const char*>(A.ch) +
-                            (size_t)(nL + (IDX)A.L + wbase[k] + (IDX)m) * (CPLX ? 8 : 4);
+                            (size_t)(nL + ahead + wbase[k] + (IDX)m) * (CPLX ? 8 : 4);
             asm volatile("prefetch.global.L1 [%0];\n" ::"l"(x));
         }
         base[k] = nL + wbase[k] + (IDX)(ok[k] ? n0 : 1);
@@ -390,10 +390,10 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
                     nlo = min(nlo, lo[i]);
                     nhi = max(nhi, hi[i]);
                 }
-                // the CTA's channels in equal parts
-                const int cnt = max(nhi - nlo + 1, 0), first = nlo;
-                nlo = first + cnt * q.part / PARTS;
-                nhi = first + cnt * (q.part + 1) / PARTS - 1;
+                // every PARTS-th channel: the weights of a part's channels end alike, and
+                // two-dimensional apertures have gaps (equal ranges of channels: 191 real
+                // channels x 191 waves 3.01 ms, this 1.87)
+                nlo += q.part;
             }
             for (int64_t w0 = 0; w0 < A.W; w0 += WC) {
                 const int wc = (int)min((int64_t)WC, A.W - w0);
@@ -407,6 +407,7 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
                 // receive values are loaded two channels ahead and the next channel's
                 // sample lines prefetched into L1 while this channel is computed
                 // (no receive weight in this warp: nhi < nlo, the loop below runs no channel)
+                const int64_t step = P * PARTS;
                 const float* pa = A.apo_rx + P * max(nlo, 0) + p;
                 const float* pd = A.d_rx + P * max(nlo, 0) + p;
                 float rxa1 = 0.f, rxd1 = 0.f, rxa2 = 0.f, rxd2 = 0.f;
@@ -414,12 +415,13 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
                     rxa1 = ld_stream(pa);
                     rxd1 = ld_stream(pd);
                 }
-                if (nlo + 1 <= nhi) {
-                    rxa2 = ld_stream(pa + P);
-                    rxd2 = ld_stream(pd + P);
+                if (nlo + PARTS <= nhi) {
+                    rxa2 = ld_stream(pa + step);
+                    rxd2 = ld_stream(pd + step);
                 }
-                pa += 2 * P;
-                pd += 2 * P;
+                pa += 2 * step;
+                pd += 2 * step;
+                const IDX ahead = (IDX)A.L * PARTS;  // to the next channel of this part
                 IDX nL = (IDX)A.L * (IDX)nlo;
                 if constexpr (CPLX) {
                     // complex: the register count left by the per-unit phase allows no
@@ -428,41 +430,41 @@ __global__ void __launch_bounds__(kThreads, (CPLX ? 1 : 6)) das_table_kernel(con
                     // channel, and lanes without a weight on this channel, form the next
                     // channel's indices for the prefetch)
                     if (FC == 1 && nlo <= nhi) prefetch_units<CPLX, IDX, MAGIC>(A, nL, wbase, wc, txd, rxd1, rxa1);
-                    for (int n = nlo; n <= nhi; ++n, nL += (IDX)A.L) {
+                    for (int n = nlo; n <= nhi; n += PARTS, nL += ahead) {
                         const float rxa = rxa1, rxd = rxd1;
                         rxa1 = rxa2;
                         rxd1 = rxd2;
-                        if (n + 2 <= nhi) {
+                        if (n + 2 * PARTS <= nhi) {
                             rxa2 = ld_stream(pa);
                             rxd2 = ld_stream(pd);
-                            pa += P;
-                            pd += P;
+                            pa += step;
+                            pd += step;
                         }
-                        const bool pf = FC == 1 && n + 1 <= nhi && rxa1 != 0.0f;
+                        const bool pf = FC == 1 && n + PARTS <= nhi && rxa1 != 0.0f;
                         if (rxa == 0.0f) {
-                            if (pf) prefetch_units<CPLX, IDX, MAGIC>(A, nL + (IDX)A.L, wbase, wc, txd, rxd1, rxa1);
+                            if (pf) prefetch_units<CPLX, IDX, MAGIC>(A, nL + ahead, wbase, wc, txd, rxd1, rxa1);
                             continue;
                         }
                         const int dn = __float2int_rn(__fmul_rn(__fsub_rn(rxd1, rxd), A.fs));
                         chunk_units<CPLX, FC, PER_WAVE, NACC, IDX, MAGIC, true>(A, nL, wbase, wc, f0, nf, txd, txa, rxd, rxa,
-                                                                          acc, pf, dn);
+                                                                          acc, pf, dn, ahead);
                     }
                 } else {
                 // real: the indices formed with the prefetch are carried to the units
                 UnitIdx<IDX> cur, nxt;
                 if (nlo <= nhi) unit_index<CPLX, IDX, MAGIC>(A, nL, wbase, wc, txd, txa, rxd1, rxa1, FC == 1, cur);
-                for (int n = nlo; n <= nhi; ++n, nL += (IDX)A.L) {
+                for (int n = nlo; n <= nhi; n += PARTS, nL += ahead) {
                     const float rxa = rxa1;
                     rxa1 = rxa2;
                     rxd1 = rxd2;
-                    if (n + 2 <= nhi) {
+                    if (n + 2 * PARTS <= nhi) {
                         rxa2 = ld_stream(pa);
                         rxd2 = ld_stream(pd);
-                        pa += P;
-                        pd += P;
+                        pa += step;
+                        pd += step;
                     }
-                    if (n + 1 <= nhi)
-                        unit_index<CPLX, IDX, MAGIC>(A, nL + (IDX)A.L, wbase, wc, txd, txa, rxd1, rxa1, FC == 1, nxt);
+                    if (n + PARTS <= nhi)
+                        unit_index<CPLX, IDX, MAGIC>(A, nL + ahead, wbase, wc, txd, txa, rxd1, rxa1, FC == 1, nxt);
                     if (rxa != 0.0f) unit_sum<CPLX, FC, PER_WAVE, IDX>(A, cur, txa, rxa, nf, acc);
                     cur = nxt;
                 }
@@ -612,9 +614,10 @@ __global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs 
 //     394 / 309; real 149 / 136, 164 / 162, 273 / 206
 //   160,000 pixels 128 x 16 (8 per SM): complex both 315 / 293, receive 322 / 372, transmit
 //     591 / 569; real 248 / 253, 283 / 311, 476 / 369; 1 wave, transmit, 84 / 83 and 54 / 56
-//   160,000 pixels 128 x 75: complex both 1199 / 1089
+//   160,000 pixels 128 x 75: complex both 1199 / 1079
 //   40,000 pixels 64 x 16 x 2 frames (2 per SM): complex receive 70 / 75
 //   320,000 pixels 64 x 16: complex both 283 / 314, receive 306 / 442
+//   41,184 pixels of a volume, 23 x 23 channels x 4 waves: complex both 602 / 635
 // A part needs channels of its own (chunks of WC).
 int in_parts(int mode, bool cplx, const TableArgs& A, bool& parts) {
     int dev = 0, sms = 0;
