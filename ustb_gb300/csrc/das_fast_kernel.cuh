@@ -18,8 +18,9 @@
 //
 // A pre-pass (build_entries_kernel) rewrites the channel data, whatever its
 // storage type, as FP32 interpolation entries {x_i, x_{i+1} - x_i} with das_c's
-// validity rule (0 < i < L-1) folded in as zero entries.  A stage's windows are
-// then plain runs of 16-byte (complex) or 8-byte (real) entries that the CTA
+// validity rule (0 < i < L-1) folded in as zero entries; complex 16-bit data keeps pairs
+// {x_i, x_{i+1}} as stored (entries_for in das_fast.cu).  A stage's windows are then plain
+// runs of 16-byte (complex FP32) or 8-byte entries that the CTA
 // copies with cp.async into one of two shared-memory buffers while it computes
 // the stage before; no per-sample work is left in the staging.  A unit costs:
 //   s = s_tx_loc + s_rx_loc; j = floor(s); b = s - j; e = slot[j];
