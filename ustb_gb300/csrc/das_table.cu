@@ -617,7 +617,9 @@ __global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs 
 //   160,000 pixels 128 x 75: complex both 1199 / 1079
 //   40,000 pixels 64 x 16 x 2 frames (2 per SM): complex receive 70 / 75
 //   320,000 pixels 64 x 16: complex both 283 / 314, receive 306 / 442
-//   41,184 pixels of a volume, 23 x 23 channels x 4 waves: complex both 602 / 635
+// Complex both of up to 12 waves stays in one part where all its CTAs are resident in one
+// full round (2 to 4 per SM): 41,184 pixels of a volume, 529 channels x 4 waves, 598 / 631;
+// 45,450 pixels 41 x 10 x 2 frames 137 / 144; 74,572 pixels 58 x 4 67 / 70.
 // A part needs channels of its own (chunks of WC).
 int in_parts(int mode, bool cplx, const TableArgs& A, bool& parts) {
     int dev = 0, sms = 0;
@@ -627,7 +629,9 @@ int in_parts(int mode, bool cplx, const TableArgs& A, bool& parts) {
     const int64_t per_sm = mode == USTB_DIM_RECEIVE && !few                                             ? 2
                            : (mode == USTB_DIM_BOTH && cplx) || (mode == USTB_DIM_TRANSMIT && !few) ? 9
                                                                                                         : 5;
-    parts = A.N >= 4 * WC && A.P <= per_sm * sms * kThreads;
+    const int64_t ctas = (A.P + kThreads - 1) / kThreads;
+    const bool one_round = mode == USTB_DIM_BOTH && cplx && !few && A.W <= 12 && ctas > 2 * sms && ctas <= 4 * sms;
+    parts = A.N >= 4 * WC && ctas <= per_sm * sms && !one_round;
     return USTB_OK;
 }
 
