@@ -87,9 +87,10 @@ __device__ __forceinline__ float rsqrt_approx(float v) {
 // value's octant; CUDA's functions for zero, infinite and NaN values and for magnitudes
 // whose squares leave the range.
 __device__ __forceinline__ void polar_of(float2 v, float& phi, float& cs, float& sn) {
-    const float ax = fabsf(v.x), ay = fabsf(v.y), hi = fmaxf(ax, ay), lo = fminf(ax, ay);
-    if (hi > 1e-18f && hi < 1e18f) {
-        const float t = lo * rcp_approx(hi), u = t * t;
+    const float n2 = fmaf(v.x, v.x, v.y * v.y);
+    if (n2 > 1e-36f && n2 < 1e36f) {
+        const float ax = fabsf(v.x), ay = fabsf(v.y);
+        const float t = fminf(ax, ay) * rcp_approx(fmaxf(ax, ay)), u = t * t;
         float q = 0.0028662257f;
         q = fmaf(q, u, -0.0161657367f);
         q = fmaf(q, u, 0.0429096138f);
@@ -102,7 +103,7 @@ __device__ __forceinline__ void polar_of(float2 v, float& phi, float& cs, float&
         r = ay > ax ? 1.57079632679f - r : r;
         r = v.x < 0.f ? kPi - r : r;
         phi = copysignf(r, v.y);
-        const float inv = rsqrt_approx(fmaf(v.x, v.x, v.y * v.y));
+        const float inv = rsqrt_approx(n2);
         cs = v.x * inv;
         sn = v.y * inv;
     } else {
