@@ -1,4 +1,4 @@
-"""Phase coherence factors of values that are not numbers, against
+"""Phase coherence factors of values that are not numbers and of tapered weights, against
 the FP64 oracle at the bar of the kernel's other tests."""
 import numpy as np
 import pytest
@@ -31,3 +31,21 @@ def test_values_that_are_not_numbers(cuda_dev, bad, weighted):
     want_a, want_c, _ = O.phase_coherence_factor_f64(c.T, None if w is None else w.T)
     assert np.array_equal(np.isnan(fcc), np.isnan(want_c)) and np.isnan(want_c).sum() == K
     assert np.max(np.abs(fca - want_a)) <= 1e-4
+
+
+@pytest.mark.parametrize("light, spread", [(1e-3, 1e-3), (1e-5, 1e-3), (1e-7, 1e-3), (1e-7, 1e-4)])
+@pytest.mark.parametrize("edge", [1, 4, 16])
+def test_light_edges_away_from_the_rest(cuda_dev, edge, light, spread):
+    """Phases that agree but for the aperture's edges, whose weights are small (a taper)."""
+    rng = np.random.default_rng(edge)
+    K, P = 64, 130
+    ang = 1.0 + spread * rng.standard_normal((K, P))
+    w = np.ones((K, P), np.float32)
+    for k in (slice(0, edge), slice(K - edge, K)):
+        ang[k] = -1.8
+        w[k] = light
+    c = np.exp(1j * ang).astype(np.complex64)
+    fca, fcc = factors(c, w, cuda_dev)
+    want_a, want_c, _ = O.phase_coherence_factor_f64(c.T, w.T.astype(np.float64))
+    assert np.max(np.abs(fca - want_a)) <= 1e-4
+    assert np.max(np.abs(fcc - want_c)) <= 1e-4

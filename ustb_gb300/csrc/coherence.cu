@@ -8,13 +8,12 @@
 //   std(x) = sqrt(sum w (x - mean_w x)^2 / sum w)     (tools/weigthed_std.m)
 //   FCA = max(0, 1 - gamma / sigma0 * min(std phi, std psi))   (NaN -> 0)
 //   FCC = 1 - sqrt(var_w(cos phi) + var_w(sin phi)),  image = FCC * sum s
-// computed in one pass, four threads per pixel over a quarter of the K values each: every
-// statistic's weighted sums of (x - x_0) and (x - x_0)^2 about the part's first value x_0
-// (no division per value, and little cancellation where the phases agree), turned into
-// mean and squared deviations and merged pairwise.  cos phi and sin phi are s / |s|, and
-// phi a short polynomial, so a value costs a division and a reciprocal square root.  GB300, 131072 pixels x 64 channels
-// with weights (100 MB): 35 us; 51 us with incremental updates (a division each) and
-// sincosf of the angle.
+// computed in one pass with weighted incremental updates (the reference's
+// mean-then-variance to rounding; sums about a fixed value cancel where an outlier of small
+// weight, such as the edge of a taper, gives that value), four threads per pixel over a
+// quarter of the K values each, merged pairwise.  cos phi and sin phi are s / |s|, and phi a
+// short polynomial.  GB300, 131072 pixels x 64 channels with weights (100 MB): 34 us; 48 us
+// with the library's arctangent, sine and cosine.
 //
 // Generalized coherence factor (+postprocess/generalized_coherence_factor.m:66-97):
 //   GCF = sum_{k in LF} |DFT_K(s)[k]|^2 / sum_k |DFT_K(s)[k]|^2   (NaN -> 0),
@@ -42,25 +41,16 @@ constexpr float kPi = 3.14159265358979f;
 constexpr int kParts = 4;                    // threads per pixel, each over a quarter of K
 constexpr int kPix = kThreads / kParts;      // pixels per CTA (64: two warps of pixels per part)
 
-// weighted sums of deviations and squared deviations from a reference value x0
+// weighted running mean and sum of squared deviations (West's incremental update,
+// the algorithm of tools/weighted_incremental_variance.m): var = S / W; partial runs
+// merge exactly (Chan et al.'s pairwise update)
 struct WRun {
-    float x0 = 0.f, s1 = 0.f, s2 = 0.f;
-    __device__ __forceinline__ void about(float x) { x0 = x == x ? x : 0.f; }  // (a NaN is no reference)
-    __device__ __forceinline__ void add(float x, float w) {
-        const float d = x - x0, q = w * d;
-        s1 += q;
-        s2 = fmaf(q, d, s2);
+    float mean = 0.f, S = 0.f;
+    __device__ __forceinline__ void add(float x, float w, float w_over_W) {
+        const float d = x - mean;
+        mean = fmaf(w_over_W, d, mean);
+        S = fmaf(w * d, x - mean, S);
     }
-    // (mean, squared deviations) of the run
-    __device__ __forceinline__ float2 result(float W) const {
-        if (W == 0.f) return make_float2(0.f, 0.f);
-        const float m = s1 / W, S = fmaf(-m, s1, s2);
-        return make_float2(x0 + m, S < 0.f ? 0.f : S);  // (rounding below 0; NaN stays)
-    }
-};
-// partial runs merge exactly (Chan et al.'s pairwise update)
-struct WStat {
-    float mean, S;
     __device__ __forceinline__ void merge(float Wa, float Wb, float mb, float Sb) {
         const float Wt = Wa + Wb;
         if (Wb == 0.f) return;
@@ -126,7 +116,7 @@ __global__ void __launch_bounds__(kThreads) pcf_kernel(const float2* __restrict_
         const int64_t f = ok ? t / P : 0, p = ok ? t - f * P : 0;
         const float2* s = cube + f * K * P + p;
         float W = 0.f;
-        WRun uphi, upsi, uc, us;
+        WRun rphi, rpsi, rc, rs;
         float2 sum = make_float2(0.f, 0.f);
         if (ok) {
             constexpr int kBatch = 4;  // values loaded together
@@ -152,22 +142,15 @@ __global__ void __launch_bounds__(kThreads) pcf_kernel(const float2* __restrict_
                     float phi, cs, sn;
                     polar_of(v[b], phi, cs, sn);
                     const float psi = phi <= 0.f ? phi + kPi : phi - kPi;
-                    if (W == 0.f) {
-                        uphi.about(phi);
-                        upsi.about(psi);
-                        uc.about(cs);
-                        us.about(sn);
-                    }
                     W += w[b];
-                    uphi.add(phi, w[b]);
-                    upsi.add(psi, w[b]);
-                    uc.add(cs, w[b]);
-                    us.add(sn, w[b]);
+                    const float q = w[b] / W;  // (an approximate quotient costs accuracy: the sums amplify it)
+                    rphi.add(phi, w[b], q);
+                    rpsi.add(psi, w[b], q);
+                    rc.add(cs, w[b], q);
+                    rs.add(sn, w[b], q);
                 }
             }
         }
-        const float2 qphi = uphi.result(W), qpsi = upsi.result(W), qc = uc.result(W), qs = us.result(W);
-        WStat rphi{qphi.x, qphi.y}, rpsi{qpsi.x, qpsi.y}, rc{qc.x, qc.y}, rs{qs.x, qs.y};
         const float v11[11] = {W, rphi.mean, rphi.S, rpsi.mean, rpsi.S, rc.mean, rc.S, rs.mean, rs.S, sum.x, sum.y};
 #pragma unroll
         for (int j = 0; j < 11; ++j) red[g][j][i] = v11[j];
@@ -184,11 +167,12 @@ __global__ void __launch_bounds__(kThreads) pcf_kernel(const float2* __restrict_
                 sum.y += red[h][10][i];
             }
             const float inv = 1.f / W;  // W = 0: NaN statistics, as the reference's 0/0
-            const float sf = fminf(sqrtf(rphi.S * inv), sqrtf(rpsi.S * inv));
+            const auto spread = [](float S) { return S < 0.f ? 0.f : S; };  // (rounding below 0; NaN stays)
+            const float sf = fminf(sqrtf(spread(rphi.S) * inv), sqrtf(spread(rpsi.S) * inv));
             float a = 1.f - gamma_over_sigma * sf;
             if (a < 0.f) a = 0.f;
             if (a != a) a = 0.f;
-            const float c = 1.f - sqrtf((rc.S + rs.S) * inv);
+            const float c = 1.f - sqrtf(spread(rc.S + rs.S) * inv);
             const int64_t o = f * P + p;
             if (fca) fca[o] = a;
             if (fcc) fcc[o] = c;
