@@ -1,4 +1,7 @@
 // Error state of the C-ABI and small shared entry points.
+#include <mutex>
+#include <vector>
+
 #include "common.cuh"
 
 namespace ustb {
@@ -24,6 +27,31 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
         return USTB_E_OOM;
     }
     return USTB_E_CUDA;
+}
+
+int shared_limit(const void* kernel, size_t& limit) {
+    struct Raised {
+        const void* kernel;
+        int dev;
+        size_t limit;
+    };
+    static std::mutex mu;
+    static std::vector<Raised> raised;  // at most the library's kernels, per device
+    int dev = 0, optin = 0;
+    USTB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Raised& r : raised)
+        if (r.kernel == kernel && r.dev == dev) {
+            limit = r.limit;
+            return USTB_OK;
+        }
+    cudaFuncAttributes fa;
+    USTB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    USTB_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    limit = (size_t)optin - fa.sharedSizeBytes;
+    USTB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    raised.push_back({kernel, dev, limit});
+    return USTB_OK;
 }
 
 }  // namespace ustb

@@ -448,7 +448,11 @@ extern "C" int ustb_capon(const void* cube, const float* apodization, int64_t nz
     const int per_warp = warp_words((int)M) * (int)sizeof(float);
     const int warps = std::max(1, std::min(kWarps, 110 * 1024 / per_warp));
     const size_t smem = (size_t)warps * per_warp;
-    USTB_CUDA(cudaFuncSetAttribute(capon_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    size_t limit = 0;
+    const int rc = ustb::shared_limit((const void*)capon_kernel, limit);
+    if (rc) return rc;
+    USTB_REQUIRE(smem <= limit, USTB_E_SHAPE, "%lld channels need %zu bytes of shared memory (limit %zu)", (long long)M,
+                 smem, limit);
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + warps - 1) / warps,
                                                                           (int64_t)sms * 64));
     cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -336,13 +336,16 @@ extern "C" int ustb_generalized_coherence(const void* cube, int64_t P, int64_t K
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned grid = grid_for(P * F);
     const float2* c = static_cast<const float2*>(cube);
-    auto start = [&](auto np) {
+    auto start = [&](auto np) -> int {
         constexpr int NP = decltype(np)::value;
         const size_t smem = sizeof(float2) * (size_t)K * NP;
-        if (smem > 16384)  // beside the partial sums
-            USTB_CUDA(cudaFuncSetAttribute(gcf_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        size_t limit = 0;
+        const int rc = ustb::shared_limit((const void*)gcf_kernel<NP>, limit);
+        if (rc) return rc;
+        USTB_REQUIRE(smem <= limit, USTB_E_SHAPE, "%lld values need %zu bytes of shared memory (limit %zu)", (long long)K,
+                     smem, limit);
         gcf_kernel<NP><<<grid, kThreads, smem, s>>>(c, P, K, F, gcf, static_cast<float2*>(image));
-        return (int)USTB_OK;
+        return USTB_OK;
     };
     int rc;
     switch (M0) {

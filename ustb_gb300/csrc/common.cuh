@@ -21,6 +21,12 @@ void clear_error();
 // USTB_E_OOM for allocation failures.
 int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 
+// The most dynamic shared memory a launch of `kernel` can ask for on the current device.
+// The kernel's own limit is raised to it once per device and never lowered: it belongs to
+// the kernel, so a limit of each call's size could be lowered by another thread between a
+// call's setting it and its launch.
+int shared_limit(const void* kernel, size_t& limit);
+
 }  // namespace ustb
 
 #define USTB_CUDA(call)                                                              \

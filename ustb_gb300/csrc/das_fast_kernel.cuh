@@ -1338,14 +1338,13 @@ cudaError_t launch_dependent(K* kern, dim3 grid, size_t smem, cudaStream_t s, co
 template <int MODE, int ENT, bool EPI, int SHAPE>
 int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
     const size_t smem = smem_bytes<SHAPE>(A.N, A.W);
-    int dev = 0, optin = 0;
-    USTB_CUDA(cudaGetDevice(&dev));
-    USTB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    USTB_REQUIRE(smem <= (size_t)optin, USTB_E_SHAPE,
-                 "%lld channels / %lld waves need %zu bytes of shared memory per tile (limit %d)",
-                 (long long)A.N, (long long)A.W, smem, optin);
     auto kern = das_fast_kernel<MODE, ENT, EPI, SHAPE>;
-    USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    size_t limit = 0;
+    const int rc = shared_limit((const void*)kern, limit);
+    if (rc) return rc;
+    USTB_REQUIRE(smem <= limit, USTB_E_SHAPE,
+                 "%lld channels / %lld waves need %zu bytes of shared memory per tile (limit %zu)",
+                 (long long)A.N, (long long)A.W, smem, limit);
     dim3 grid((unsigned)(n_tiles * kSub * A.split), (unsigned)F);
     // only the pre-pass is known to leave the outputs and the geometry alone
     if (A.after_entries) {
@@ -1364,9 +1363,8 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
     B.n = n;
     B.counter = counter;
     B.first_item[0] = 0;
-    int dev = 0, optin = 0, sms = 0;
+    int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
-    USTB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t nct = (max_ctas > 0 ? std::min(max_ctas, sms) : sms) * (int64_t)kSub;
     size_t smem = 0;
@@ -1380,10 +1378,12 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
         smem = std::max(smem, smem_bytes<SHAPE>(reqs[i].N, reqs[i].W));
     }
     if (B.first_item[n] == 0) return USTB_OK;
-    USTB_REQUIRE(smem <= (size_t)optin, USTB_E_SHAPE, "a request needs %zu bytes of shared memory per tile (limit %d)",
-                 smem, optin);
     auto kern = das_fast_persistent<MODE, ENT, EPI, SHAPE>;
-    USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    size_t limit = 0;
+    const int rc = shared_limit((const void*)kern, limit);
+    if (rc) return rc;
+    USTB_REQUIRE(smem <= limit, USTB_E_SHAPE, "a request needs %zu bytes of shared memory per tile (limit %zu)", smem,
+                 limit);
     USTB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
     // two CTAs per SM, or fewer (max_ctas pairs) to leave room to launches on other streams
     const unsigned grid = (unsigned)std::min<int64_t>(B.first_item[n], nct);

@@ -435,19 +435,20 @@ int launch_demod(const S* rf, void* iq, int32_t dst_type, const float* taps, Dem
     plan_demod(a, ZP, ((uintptr_t)rf & (4 * sizeof(S) - 1)) == 0);
     USTB_REQUIRE(a.groups <= INT32_MAX, USTB_E_SHAPE, "too many traces x output chunks");
     const size_t smem = sizeof(float) * demod_layout(a, ZP).total;
-    int dev = 0, optin = 0, sms = 0;
+    int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
-    USTB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    USTB_REQUIRE(smem <= (size_t)optin, USTB_E_SHAPE, "decimation %d with %d taps needs %zu bytes of shared memory",
-                 a.D, a.ntaps, smem);
     const unsigned threads = (unsigned)((a.tp * a.tpt + 31) / 32 * 32);
     const unsigned blocks = (unsigned)std::min<int64_t>(a.groups, (int64_t)sms * 16);
-    auto start = [&](auto kern, auto* dst) {
-        USTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto start = [&](auto kern, auto* dst) -> int {
+        size_t limit = 0;
+        const int rc = ustb::shared_limit((const void*)kern, limit);
+        if (rc) return rc;
+        USTB_REQUIRE(smem <= limit, USTB_E_SHAPE, "decimation %d with %d taps needs %zu bytes of shared memory", a.D,
+                     a.ntaps, smem);
         kern<<<blocks, threads, smem, s>>>(rf, dst, taps, a);
         USTB_CUDA(cudaGetLastError());
-        return (int)USTB_OK;
+        return USTB_OK;
     };
     switch (dst_type) {
         case USTB_STORE_F32: return start(demod_kernel<S, float, ZP>, (float*)iq);
