@@ -484,6 +484,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     const int p = live ? p_own : (in_image(p_anchor) ? p_anchor : 0);
     const float* const pxyz = A.px + 3 * (int64_t)p;
     const float px = __ldg(pxyz), py = __ldg(pxyz + 1), pz = __ldg(pxyz + 2);
+    if (live && py != py) s_in_plane = 0;  // the box does not hold it: its window is 0, not 1
 
     Box box, tbox;  // sub-tile, whole tile
     {
