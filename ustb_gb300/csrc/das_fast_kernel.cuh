@@ -772,7 +772,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     float eI = 0.f, eM = 0.f, eR = 0.f, eQ = 0.f;
 
     // a channel's receive part: its place in the slot and its weight (times the phasor)
-    auto put_rx = [&](int c, float s, float2 rp, float apo) {
+    auto put_rx = [&](int c, int n, float s, float2 rp, float apo) {
         if (CPLX) {
             const float2 e = phasor_cycles(fmaf(s, fdfs, rp.x));
             B[c] = make_float2(apo * e.x, apo * e.y);
@@ -780,7 +780,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             B[c] = make_float2(apo, 0.f);
         }
         srx[c] = fminf(fmaxf(s - rp.y, 0.f), hn);  // NaN -> 0: stays inside the slot
-        if constexpr (EPI) eM += apo > A.cf_thr ? 1.f : 0.f;
+        if constexpr (EPI) eM += (n < (int)N && apo > A.cf_thr) ? 1.f : 0.f;  // (weight 0 counts below a negative threshold)
     };
     // Closed-form window (no table): the same arithmetic as rx_apodization without its
     // per-channel branches; padding channels are inactive, so their weight is 0.
@@ -815,7 +815,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
                 if (yd != 0.f) apo *= window(A, fabsf(A.fny * (yd * rcy)));
             }
             if (!live || !act_n(n)) apo = 0.f;
-            put_rx(c, s, rxp[n], apo);
+            put_rx(c, n, s, rxp[n], apo);
         }
     };
     auto setup_rx = [&](int n0) {
@@ -835,10 +835,11 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
                 const float s = (r * A.inv_c + A.lens) * A.fs - e4.w;
                 float apo = A.rx_apo_tab ? __ldg(A.rx_apo_tab + (int64_t)n * P + p) : rx_apodization(A, ex, ey, ez, px, py, pz);
                 if (!live) apo = 0.f;
-                put_rx(c, s, rxp[n], apo);
+                put_rx(c, n, s, rxp[n], apo);
             } else {
                 srx[c] = 0.f;
                 B[c] = make_float2(0.f, 0.f);
+                if constexpr (EPI) eM += (n < (int)N && 0.f > A.cf_thr) ? 1.f : 0.f;
             }
         }
     };
