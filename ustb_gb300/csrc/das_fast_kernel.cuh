@@ -365,7 +365,7 @@ __host__ __device__ __forceinline__ TileTables tile_tables(int64_t NP, int64_t W
     t.el4 = o;    o += 16 * NP;        // float4 per channel: x, y, z, delay base
     t.txc = o;    o += 16 * WP;        // float4 per wave: delay coefficients
     t.txp = o;    o += 16 * WP;        // float4 per wave: phase offset, apodization, fs/c, window offset
-    t.win_w = o;  o += 8 * WP;         // {window start, its largest position as a float (< 0: inactive)} per wave
+    t.win_w = o;  o += 8 * WP;         // {window start, its largest position as a float (sign bit: inactive)} per wave
     t.rxp = o;    o += 8 * NP;         // float2 per channel: phase (cycles) of the delay base, window offset
     t.base_w = o; o += 4 * WP;         // delay base of each wave
     t.len_n = o;  o += 4 * NP;         // largest window position of each channel (< 0: inactive)
@@ -375,8 +375,9 @@ __host__ __device__ __forceinline__ TileTables tile_tables(int64_t NP, int64_t W
     return t;
 }
 
-// Once per CTA: zero the stage buffers, so that units with zero weight, which may read
-// past a window's end, never read uninitialised words.  The caller's barriers follow.
+// Once per CTA: zero the stage buffers, so that units whose sums nothing takes (idle lanes,
+// inactive channels), which may read past a window's end, never read uninitialised words.
+// The caller's barriers follow.
 __device__ __forceinline__ void zero_slots() {
     extern __shared__ __align__(16) unsigned char smem[];
     float4* z = reinterpret_cast<float4*>(smem);
@@ -511,7 +512,10 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
 
     // ---- per-tile delay bases, window parts, activity and delay/phase coefficients ----
     const double fd_fs = A.fd_fs;
-    const int2 inactive = make_int2(0, __float_as_int(-1e9f));
+    // Padding waves have no window.  The units of a wave without a weight are evaluated, so
+    // it has one that lies before every trace and zeros are stored for it: what an earlier
+    // stage left in its slots may not be finite.  Either length has its sign bit set.
+    const int2 inactive = make_int2(0, __float_as_int(-1e9f)), zeros = make_int2(-(1 << 30), __float_as_int(-0.f));
     auto act_n = [&](int n) { return len_n[n] >= 0.f; };
     auto act_w = [&](int w) { return win_w[w].y >= 0; };  // the sign bit
     // sub-tile delays [lo, hi] -> window start j after `base` and largest position after
@@ -589,8 +593,12 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         hi = (hi - A.t0) * A.fs;
         float j, len;
         window_part(bw, lo, hi, j, len);
-        win_w[w] = act ? pack_part(bw, j, len) : inactive;
-        if (act) longest_w = fmaxf(longest_w, len);
+        win_w[w] = act ? pack_part(bw, j, len) : zeros;
+        if (!act) {  // at position 0 of the window of zeros
+            txc[w] = txp[w] = make_float4(0.f, 0.f, 0.f, 0.f);
+            continue;
+        }
+        longest_w = fmaxf(longest_w, len);
         // s_tx(p) = (tau(p) - t0) fs - base_w; constant part in double
         const double fs_c = wv.sound_speed == A.c ? A.fs_c : (double)A.fs / (double)wv.sound_speed;
         const double c0 = -((double)wv.delay + (double)A.t0) * (double)A.fs - (double)bw;
@@ -690,14 +698,14 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     // entries outside the trace, in windows that cross one of its ends, are stored as
     // zeros.  i0 and len come from the per-tile {start, length} of the slot's channel and
     // wave.  A thread always serves the same slot (c, k), so what depends on the outer
-    // index is formed when it changes.  Slots without work (inactive channel or wave) are
-    // left as they are: their units carry zero weight and read finite stale entries.
+    // index is formed when it changes.  Slots of inactive channels and of padding are left
+    // as they are: nothing that is stored has read them.
     constexpr int NWARPS = kThreads / 32, PER = NS / NWARPS, LPS = 32 / PER;  // slots per warp, lanes per slot
     const int my_sl = warp * PER + lane / LPS, my_c = my_sl / KW, my_k = my_sl - my_c * KW, hl = lane % LPS;
     const Entry* const ent_f = reinterpret_cast<const Entry*>(A.entries) + f0 * A.frame_step;
     const uint32_t my_dst = slots_s + (uint32_t)(my_sl * SLOT + hl) * ES;
     int part_start = 0;                       // the outer index's part of my slot's window
-    float part_len = 0.f;                     // (< 0: no work)
+    float part_len = 0.f;                     // (-1e9: no work)
     const Entry* part_src = ent_f;            // entry 0 of the channel's first wave (waves outer: of channel 0's wave)
     auto chan_part = [&](int n, int& start, float& len, const Entry*& src) {
         len = len_n[n];
@@ -1163,6 +1171,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
         };
         constexpr unsigned kAll = (1u << CG) - 1u;
         constexpr int kWhole = 0, kMasked = 1, kPart = 2;
+        static_assert(KW <= 4, "only the last wave of a chunk that is more than half full can be padding");
         auto units = [&](int n0, int w0, auto all) {
             if constexpr (MODE == USTB_DIM_NONE) {
 #pragma unroll
@@ -1181,6 +1190,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
             } else if constexpr (decltype(all)::value == kWhole) {
 #pragma unroll
                 for (int k = 0; k < KW; ++k) {
+                    if (KW > 2 && k + 1 == KW && w0 + k >= W) continue;  // padding
                     const f32x2 ax = pack2(Aw[k].x, Aw[k].x), ay = pack2(Aw[k].y, Aw[k].y);
                     const f32x2 nay = pack2(-Aw[k].y, -Aw[k].y), st = pack2(stx[k], stx[k]);
 #pragma unroll
@@ -1194,7 +1204,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
                     const f32x2 sr = pack2(srx[c], srx[c + 1]);
 #pragma unroll
                     for (int k = 0; k < KW; ++k) {
-                        if (decltype(all)::value == kPart && w0 + k >= W) continue;  // padding of the last wave chunk
+                        if ((decltype(all)::value == kPart || (KW > 2 && k + 1 == KW)) && w0 + k >= W) continue;  // padding
                         unit_pair(c / 2, add2(pack2(stx[k], stx[k]), sr), c, k, c + 1, k, pack2(Aw[k].x, Aw[k].x),
                                   pack2(Aw[k].y, Aw[k].y), pack2(-Aw[k].y, -Aw[k].y));
                     }
