@@ -243,9 +243,10 @@ typedef struct {
  * flags: device uint32, cleared by the call; USTB_FLAG_WINDOW_OVERFLOW means a
  * tile was too large for its sample windows (re-plan with smaller tiles).
  * The call first rewrites the channel data as FP32 interpolation entries
- * {x_i, x_(i+1) - x_i} (16 bytes per complex sample, 8 per real one) in a
- * stream-ordered scratch array that the library allocates from its own memory
- * pool and frees before returning (USTB_E_OOM when it does not fit).
+ * {x_i, x_(i+1) - x_i} (16 bytes per complex sample, 8 per real one), or complex 16-bit
+ * data as pairs {x_i, x_(i+1)} in its storage type (8 bytes), in a stream-ordered
+ * scratch array that the library allocates from its own memory pool and frees before
+ * returning (USTB_E_OOM when it does not fit).
  */
 int ustb_das_fast(const void* ch, int32_t storage, int32_t is_complex, int64_t L, int64_t N,
                   int64_t W, int64_t F, const ustb_das_geometry* geometry, int32_t dimension,
@@ -283,8 +284,10 @@ typedef struct {
  * Batched, persistent form of ustb_das_fast: every request is cut into
  * (frame, tile) work items and two CTAs per SM pull items from a queue until all
  * are done, so requests of different scans, probes, frame counts and sizes share
- * one launch and balance across the GPU (one launch per kernel variant, i.e. per
- * dimension / real-complex / epilogue combination present).  Each request's
+ * one launch and balance across the GPU (one launch per dimension / real-complex /
+ * epilogue combination and stage_shape present; batches of more than 16 work items per
+ * persistent CTA also launch once per kind of entries and of receive stages, which differ
+ * with the storage type and the number of waves).  Each request's
  * entry array (see ustb_das_fast) lives in library scratch until the launches are done.  The
  * reference runs requests one at a time (+midprocess/das.m:77-317,
  * +mex/source/das_cuda.cu:253-283 pipelines only frames).
@@ -295,8 +298,8 @@ typedef struct {
 int ustb_das_fast_batch(const ustb_das_request* reqs, int32_t n, uint64_t* scratch, void* stream);
 
 /*
- * Device bytes that ustb_das_fast_batch_ws needs as workspace for this batch:
- * the FP32 interpolation entries of every request, each on a 256-byte boundary.
+ * Device bytes that ustb_das_fast_batch_ws needs as workspace for this batch: room for
+ * FP32 interpolation entries of every request, each on a 256-byte boundary.
  * No reference counterpart (the reference keeps no device working set).
  */
 int64_t ustb_das_fast_workspace_bytes(const ustb_das_request* reqs, int32_t n);

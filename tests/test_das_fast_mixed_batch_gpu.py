@@ -1,0 +1,62 @@
+"""Batches whose requests differ in storage type and number of waves: one launch while they
+are few, and every request's own result (the batch's persistent kernel against a launch of
+its own; 1e-6 leaves room for another order of the sums)."""
+import numpy as np
+import pytest
+import torch
+
+from ustb_gb300 import fast
+from ustb_gb300.enums import Precision, Window
+from ustb_gb300.geometry import Apodization
+from ustb_gb300.uff import LinearScan, Probe, Wave
+
+pytestmark = pytest.mark.gpu
+
+L, FS, F0, T0 = 400, 20e6, 5e6, 2e-6
+
+
+def request(rng, precision, W, cplx, dim, epi, dev, F=1, shape=0):
+    N = 18
+    seq = [Wave.plane(float(a)) for a in np.deg2rad(np.linspace(-9, 9, W))]
+    scan = LinearScan(np.linspace(-3e-3, 3e-3, 23), np.linspace(6e-3, 11e-3, 47))
+    rx = Apodization(window=Window.tukey25, f_number=1.2)
+    g = fast.FastGeometry(Probe.linear_array(N, 0.3e-3), scan, seq, FS, T0, F0 if cplx else 0.0, 1540.0, dev, rx, None,
+                          stage_shape=shape)
+    x = rng.standard_normal((F, W, N, L) + ((2,) if cplx else ())).astype(np.float32)
+    st = torch.from_numpy(x).to(dev).to(fast.TORCH_STORE[precision])
+    return fast.Request(st, precision, cplx, g, dim, F=F, L=L, epilogue=epi)
+
+
+def launches(scratch):
+    return int((scratch[1:] != 0).sum())  # each launch has its own queue counter
+
+
+@pytest.mark.parametrize("workspace", [False, True])
+@pytest.mark.parametrize("dim, cplx, epi", [(3, True, False), (3, False, False), (2, True, False), (2, True, True),
+                                            (1, True, False), (1, False, False), (0, True, False)])
+def test_few_items_share_a_launch(cuda_dev, dim, cplx, epi, workspace):
+    rng = np.random.default_rng(dim)
+    reqs = [request(rng, p, W, cplx, dim, epi, cuda_dev, F=1 + W % 2)
+            for p in (Precision.fp16, Precision.fp32, Precision.bf16) for W in (1, 2, 5, 11)]
+    ws = torch.empty(fast.workspace_bytes(reqs), dtype=torch.uint8, device=cuda_dev) if workspace else None
+    scratch = fast.das_fast_batch(reqs, workspace=ws)
+    assert launches(scratch) == 1 and int(scratch[0]) == 0
+    for r in reqs:
+        alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, dim, F=r.F, L=L, epilogue=epi)
+        for k, y in r.outputs.items():
+            ok = torch.isfinite(alone[k].abs())  # a factor is infinite where no weight exceeds the threshold
+            assert torch.equal(ok, torch.isfinite(y.abs()))
+            assert torch.linalg.vector_norm((y - alone[k])[ok]) <= 1e-6 * torch.linalg.vector_norm(alone[k][ok]), k
+
+
+def test_stages_asked_for_stay(cuda_dev):
+    """A request with a stage shape of its own keeps it, in a launch of its own."""
+    rng = np.random.default_rng(9)
+    reqs = [request(rng, Precision.fp32, W, True, 1, False, cuda_dev, shape=s) for W, s in ((1, 0), (20, 0), (5, 1))]
+    assert launches(fast.das_fast_batch(reqs)) == 2
+
+
+def test_many_items_keep_their_variants(cuda_dev):
+    rng = np.random.default_rng(9)
+    reqs = [request(rng, p, 1 + i % 2 * 3, True, 1, False, cuda_dev, F=600) for i in range(2) for p in (Precision.fp32,)]
+    assert launches(fast.das_fast_batch(reqs)) == 2

@@ -477,6 +477,47 @@ extern "C" int ustb_das_fast_entries(const void* entries, int32_t is_complex, in
     return USTB_OK;
 }
 
+// Requests of one dimension, data kind and epilogue whose variants differ only by the
+// library's choices (entries in the storage type, receive stages by the number of waves)
+// run as one launch, with FP32 entries and the 8 x 4 stages, while they make at most 16
+// rounds of CTAs: launches of a few rounds each leave SMs idle one after the other, and in
+// longer ones the variants' own speed weighs more.  Measured, a launch per variant / one:
+// six requests of FP32, FP16 and bfloat16 data, 11 waves, on 64 x 64 pixels 194 / 124 us, on
+// 128 x 128 (1.3 rounds) 349 / 210, 31 waves on 256 x 256 (5 rounds) 657 / 650, twelve of
+// them (10 rounds) 1236 / 1257, six on 400 x 400 (12 rounds) 1196 / 1182; receive images of 1,
+// 4 and 20 waves on 64 x 64 182 / 142, on 200 x 200 in the three types 461 / 362.
+constexpr int64_t kShareRounds = 16;
+static int share_variants(const ustb_das_request* reqs, int32_t n, const std::vector<int>& key, std::vector<Params>& P) {
+    int dev = 0, sms = 0;
+    USTB_CUDA(cudaGetDevice(&dev));
+    USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    for (int dim = 0; dim < 4; ++dim)
+        for (int epi = 0; epi < 2; ++epi)
+            for (int cplx = 0; cplx < 2; ++cplx) {
+                auto member = [&](int i) {
+                    const ustb_das_request& q = reqs[i];
+                    return key[i] >= 0 && q.dimension == dim && (q.epilogue != 0) == (epi != 0) && q.is_complex == cplx &&
+                           q.geometry->stage_shape == 0;
+                };
+                int first = -1;
+                bool differ = false;
+                int64_t items = 0;  // half tiles x frames
+                for (int i = 0; i < n; ++i) {
+                    if (!member(i)) continue;
+                    if (first < 0) first = i;
+                    differ |= P[i].ent != P[first].ent || P[i].shape != P[first].shape;
+                    items += P[i].n_tiles * ustb::kSub * P[i].F;
+                }
+                if (!differ || items > kShareRounds * ustb::kSub * sms) continue;
+                for (int i = 0; i < n; ++i) {
+                    if (!member(i)) continue;
+                    if (cplx) P[i].ent = ustb::kEntComplex;
+                    if (dim == USTB_DIM_RECEIVE) P[i].shape = 3;
+                }
+            }
+    return USTB_OK;
+}
+
 static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t* scratch, void* workspace,
                                int64_t workspace_bytes, int32_t max_ctas, void* stream) {
     ustb::clear_error();
@@ -503,8 +544,12 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
             return rc;
         }
         frames[i] = q.F;
-        if (!empty) key[i] = ((q.dimension * 4 + P[i].ent) * 2 + (q.epilogue ? 1 : 0)) * 8 + P[i].shape;
+        if (!empty) key[i] = 0;
     }
+    int rc = share_variants(reqs, n, key, P);
+    if (rc) return rc;
+    for (int i = 0; i < n; ++i)
+        if (key[i] >= 0) key[i] = ((reqs[i].dimension * 4 + P[i].ent) * 2 + (reqs[i].epilogue ? 1 : 0)) * 8 + P[i].shape;
     // every request's entry array: carved from the caller's workspace, or allocated
     // from the library pool and freed (stream-ordered) after the launches
     std::vector<void*> ents;
