@@ -201,8 +201,9 @@ typedef struct {
     int32_t rx_use_origin;       /* 0: aperture centred under each pixel; 1: at rx_origin (sector scans) */
     float rx_origin[3];
     float cf_threshold;          /* coherence factor: elements with rx apodization > this count in M */
-    int32_t ctas_per_tile;       /* dimension.both, one launch per request: 1 to 4 CTAs per half tile,
-                                    each over an equal part of its stages; the last to finish adds
+    int32_t ctas_per_tile;       /* dimension.both, one launch per request: 1 to 4 CTAs per half tile
+                                    (per tile, where the tables of about 1180 channels or more leave
+                                    room for one CTA on an SM), each over an equal part of its stages; the last to finish adds
                                     their sums in order, so repeated runs give the same bits.  0 = the
                                     library picks from the numbers of tiles and stages, up to 8;
                                     transmit and receive split the same way and ignore this */
@@ -282,7 +283,7 @@ typedef struct {
 
 /*
  * Batched, persistent form of ustb_das_fast: every request is cut into
- * (frame, tile) work items and two CTAs per SM pull items from a queue until all
+ * (frame, tile) work items and the CTAs that fit the SMs pull items from a queue until all
  * are done, so requests of different scans, probes, frame counts and sizes share
  * one launch and balance across the GPU (one launch per dimension / real-complex /
  * epilogue combination and stage_shape present; batches of more than 16 work items per
@@ -317,7 +318,7 @@ int ustb_das_fast_batch_ws(const ustb_das_request* reqs, int32_t n, uint64_t* sc
 
 /*
  * ustb_das_fast_batch / _ws with a bound on the persistent launch's CTAs:
- * max_ctas > 0 takes at most the room of that many whole SMs (two half-SM CTAs each),
+ * max_ctas > 0 takes at most the room of that many whole SMs (two half-SM CTAs each, or one),
  * leaving the rest to launches on other streams, e.g. small requests served while a
  * large one runs; 0 = every SM.  workspace may be NULL (library pool, as
  * ustb_das_fast_batch).  No reference counterpart (the reference serves nothing).

@@ -9,6 +9,16 @@
 
 #include "das_fast.cuh"
 
+int ustb::ctas_per_sm(size_t smem, int& n) {
+    int dev = 0, per_sm = 0, reserved = 0;
+    USTB_CUDA(cudaGetDevice(&dev));
+    USTB_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    USTB_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+    constexpr size_t kStatic = 512;  // the kernels' static shared memory at most
+    n = 2 * (smem + kStatic + (size_t)reserved) <= (size_t)per_sm ? 2 : 1;
+    return USTB_OK;
+}
+
 namespace {
 
 using ustb::kMaxBatch;
@@ -67,7 +77,7 @@ int shape_for(int dim, bool cplx, int32_t requested, int64_t W) {
 // transmit and receive split where their outputs do not overlap; the epilogue's sums over
 // channels are added like dimension.both's (81 channels x 29 waves into 68 x 89 pixels with
 // coherence factors: one part 159 us, three 78).
-int parts_for(const Params& A, int dim, bool epi, int32_t requested, int& parts) {
+int parts_for(const Params& A, int dim, int32_t requested, int& parts) {
     parts = 1;
     if (dim == USTB_DIM_BOTH && requested > 0) {
         parts = requested;
@@ -77,21 +87,37 @@ int parts_for(const Params& A, int dim, bool epi, int32_t requested, int& parts)
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    constexpr int kCG[6] = {2, 8, 16, 8, 16, 4}, kKW[6] = {16, 4, 2, 4, 2, 8};
-    const int64_t groups = (A.N + kCG[A.shape] - 1) / kCG[A.shape], chunks = (A.W + kKW[A.shape] - 1) / kKW[A.shape];
+    const ustb::StageShape sh = ustb::kShapes[A.shape];
+    const int64_t groups = (A.N + sh.cg - 1) / sh.cg, chunks = (A.W + sh.kw - 1) / sh.kw;
     const int64_t most = dim == USTB_DIM_RECEIVE ? chunks : dim == USTB_DIM_TRANSMIT ? groups : groups * chunks / 4;
     const double stages = (double)groups * (double)chunks;
     const double setup = 4.5 + (double)(A.N + A.W) / 128.0;  // of a CTA, in stages
-    const double rounds = (double)A.n_tiles * ustb::kSub * (double)A.F / (2.0 * sms);  // of one part each
+    const double rounds = (double)A.n_tiles * (double)A.F / sms;  // of one part each (A.subs CTAs per SM)
     double best = 0.0;
     for (int k = 1; k <= 8 && k <= most; ++k) {
-        const double r = std::max(k * rounds, 0.5), uneven = 0.25 + 0.5 * std::min(std::max(1.5 - r, 0.0), 0.5);
+        const double r = std::max(k * rounds, 1.0 / A.subs), uneven = 0.25 + 0.5 * std::min(std::max(1.5 - r, 0.0), 0.5);
         const double cost = (r + uneven) * (setup + stages / k);
         if (k == 1 || cost < 0.99 * best) {
             parts = k;
             best = cost;
         }
     }
+    return USTB_OK;
+}
+
+// Sub-tiles per tile: two CTAs of half a tile share an SM.  Where a request's tables leave
+// room for one CTA (from about 1180 channels with a few waves, 970 with 128), dimension.both
+// takes the whole tile with twice the threads, and FP32 entries.  Half / whole tiles, us:
+// 35 x 35 elements x 9 waves on 32 x 32 x 48 pixels 662 / 460, on 16 x 16 x 48 257 / 205, 48 x 48
+// real x 4 waves 406 / 283, 1024 x 128 half-precision 2687 / 2459.  Transmit and receive
+// images keep halves: 35 x 35 x 4 waves on 24 x 24 x 32 354 / 367; receive, 9 waves on
+// 32 x 32 x 48, 653 / 708, 48 x 48 real x 2 waves 333 / 417.
+int subs_for(Params& A, int dim) {
+    int fit = 0;
+    const int rc = ustb::ctas_per_sm(ustb::smem_bytes(A.shape, A.N, A.W), fit);
+    if (rc) return rc;
+    A.subs = dim == USTB_DIM_BOTH && fit == 1 ? 1 : 2;
+    if (A.subs == 1 && A.ent != ustb::kEntReal) A.ent = ustb::kEntComplex;
     return USTB_OK;
 }
 
@@ -257,8 +283,8 @@ int build_entries(const void* ch, int32_t storage, int ent_kind, int64_t L, int6
 int64_t part_bytes(const Params& A, int dim, bool epi, int64_t& tickets) {
     tickets = 0;
     if (A.split <= 1 || (dim != USTB_DIM_BOTH && !epi)) return 0;
-    tickets = A.n_tiles * ustb::kSub * A.F;
-    return tickets * A.split * ustb::kThreads * (epi ? 3 : 1) * (int64_t)sizeof(float2);
+    tickets = A.n_tiles * A.subs * A.F;
+    return tickets * A.split * (ustb::kTile / A.subs) * (epi ? 3 : 1) * (int64_t)sizeof(float2);
 }
 void set_parts(Params& A, void* scratch, int64_t sums) {
     A.partial = static_cast<float2*>(scratch);
@@ -270,8 +296,11 @@ template <bool BATCH>
 int dispatch(int dim, int epi, const Params* reqs, const int64_t* frames, int n, unsigned long long* counter,
              int64_t nt, int64_t F, cudaStream_t s, int max_ctas) {
     auto run = [&](auto ent) {
-        return ustb::das_dispatch<decltype(ent)::value, BATCH>(dim, epi, reqs[0].shape, reqs, frames, n, counter, nt, F, s,
-                                                               max_ctas);
+        constexpr int ENT = decltype(ent)::value;
+        if constexpr (ENT == ustb::kEntReal || ENT == ustb::kEntComplex)
+            if (reqs[0].subs == 1)
+                return ustb::das_dispatch<ENT, BATCH, 1>(dim, epi, reqs[0].shape, reqs, frames, n, counter, nt, F, s, max_ctas);
+        return ustb::das_dispatch<ENT, BATCH, 2>(dim, epi, reqs[0].shape, reqs, frames, n, counter, nt, F, s, max_ctas);
     };
     switch (reqs[0].ent) {
         case ustb::kEntReal: return run(std::integral_constant<int, ustb::kEntReal>{});
@@ -382,8 +411,9 @@ static int make_params(const void* ch, int32_t storage, int32_t is_complex, int6
                  (int)g->stage_shape, (int)dimension);
     A.shape = shape_for(dimension, is_complex != 0, g->stage_shape, W);
     A.ent = entries_for(storage, is_complex != 0, dimension, A.shape, W);
-    A.split = 1;
-    const int rc = parts_for(A, dimension, epilogue != 0, g->ctas_per_tile, A.split);
+    int rc = subs_for(A, dimension);
+    if (rc) return rc;
+    rc = parts_for(A, dimension, g->ctas_per_tile, A.split);
     if (rc) return rc;
     A.fpi = 1;
     return USTB_OK;
@@ -486,6 +516,9 @@ extern "C" int ustb_das_fast_entries(const void* entries, int32_t is_complex, in
 // 128 x 128 (1.3 rounds) 349 / 210, 31 waves on 256 x 256 (5 rounds) 657 / 650, twelve of
 // them (10 rounds) 1236 / 1257, six on 400 x 400 (12 rounds) 1196 / 1182; receive images of 1,
 // 4 and 20 waves on 64 x 64 182 / 142, on 200 x 200 in the three types 461 / 362.
+// Whole tiles (subs_for) need enough of them here, where no parts fill the SMs: 35 x 35
+// elements x 4 waves with 3 requests of 64 elements, 64 tiles, 576 us as halves, 846 whole;
+// 9 waves, 256 tiles, 3138 / 2808.
 constexpr int64_t kShareRounds = 16;
 static int share_variants(const ustb_das_request* reqs, int32_t n, const std::vector<int>& key, std::vector<Params>& P) {
     int dev = 0, sms = 0;
@@ -501,16 +534,22 @@ static int share_variants(const ustb_das_request* reqs, int32_t n, const std::ve
                 };
                 int first = -1;
                 bool differ = false;
-                int64_t items = 0;  // half tiles x frames
+                int64_t items = 0, whole = 0;  // tiles x frames; of requests that take whole tiles
                 for (int i = 0; i < n; ++i) {
                     if (!member(i)) continue;
                     if (first < 0) first = i;
-                    differ |= P[i].ent != P[first].ent || P[i].shape != P[first].shape;
-                    items += P[i].n_tiles * ustb::kSub * P[i].F;
+                    differ |= P[i].ent != P[first].ent || P[i].shape != P[first].shape || P[i].subs != P[first].subs;
+                    items += P[i].n_tiles * P[i].F;
+                    if (P[i].subs == 1) whole += P[i].n_tiles * P[i].F;
                 }
-                if (!differ || items > kShareRounds * ustb::kSub * sms) continue;
+                // too few whole tiles for every SM: halves go to twice as many
+                const int subs = whole > sms / 2 ? 1 : 2;
+                for (int i = 0; i < n; ++i)
+                    if (member(i)) P[i].subs = std::max(P[i].subs, subs);
+                if (!differ || items > kShareRounds * sms) continue;
                 for (int i = 0; i < n; ++i) {
                     if (!member(i)) continue;
+                    P[i].subs = subs;
                     if (cplx) P[i].ent = ustb::kEntComplex;
                     if (dim == USTB_DIM_RECEIVE) P[i].shape = 3;
                 }
@@ -549,7 +588,8 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
     int rc = share_variants(reqs, n, key, P);
     if (rc) return rc;
     for (int i = 0; i < n; ++i)
-        if (key[i] >= 0) key[i] = ((reqs[i].dimension * 4 + P[i].ent) * 2 + (reqs[i].epilogue ? 1 : 0)) * 8 + P[i].shape;
+        if (key[i] >= 0)
+            key[i] = (((reqs[i].dimension * 4 + P[i].ent) * 2 + (reqs[i].epilogue ? 1 : 0)) * 8 + P[i].shape) * 2 + P[i].subs - 1;
     // every request's entry array: carved from the caller's workspace, or allocated
     // from the library pool and freed (stream-ordered) after the launches
     std::vector<void*> ents;

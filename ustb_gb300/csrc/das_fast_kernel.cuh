@@ -10,7 +10,8 @@
 //
 // One CTA of 256 threads beamforms half of a 512-pixel tile (one pixel per thread) for
 // one frame; two CTAs share an SM, so that one computes while the other waits at a stage
-// barrier or sets a tile up.  The (channel, wave) pairs are processed in stages of 32
+// barrier or sets a tile up.  (Tables of about 1180 channels or more leave room for one: then
+// a CTA of 512 threads may take the whole tile, see subs_for in das_fast.cu.)  The (channel, wave) pairs are processed in stages of 32
 // slots; for each pair the CTA needs a short window of samples whose start and length
 // follow from bounding boxes: the delay bases base_n / base_w are integer lower bounds of
 // the whole tile's receive / transmit delays (in samples), the windows cover the CTA's
@@ -60,10 +61,14 @@
 namespace ustb {
 namespace {
 
-static_assert(kTile == kSub * kThreads, "a CTA takes one sub-tile, one pixel per thread");
-constexpr int kBufBytes = 40960;                // a stage buffer: 32 slots x 80 or 16 x 160 complex entries, 32 x 160 real
+// Sub-tiles (CTAs) per tile, set by the including file: 2, or 1 for requests whose tables
+// leave no room for two CTAs on an SM.
+#ifndef USTB_SUBS
+#define USTB_SUBS 2
+#endif
+constexpr int kSub = USTB_SUBS;
+constexpr int kThreads = kTile / kSub;          // a CTA takes one sub-tile, one pixel per thread
 constexpr int kItemFrames = 8;                  // frames of a persistent work item at most
-constexpr int kRing = 2;                        // stage buffers: stage s + kRing - 1 is copied during stage s
 constexpr float kHalf = 79.f;                   // max relative delay of each component (160-entry slots)
 constexpr float kMagic = 8388608.0f;            // 2^23: floor via round-toward-zero add
 constexpr int kMagicBits = 0x4B000000;
@@ -290,50 +295,10 @@ __device__ __forceinline__ bool rx_active(const Params& A, const Box& b, float e
     return !(A.fnx * xd / zx > lim || A.fny * yd / zy > lim);
 }
 
-// Stage shapes: a stage is CG channels x KW waves (channel, wave) slots.
-//   shape 0: waves outer (2 channels x 16 waves); per-wave accumulators, the
-//            receive geometry of a channel is formed once per 16-wave chunk
-//   shape 1: channels outer (8 channels x 4 waves); per-channel accumulators,
-//            the receive geometry is formed once per (pixel, channel) and the
-//            transmit geometry once per stage
-//   shape 2: channels outer (16 channels x 2 waves)
-//   shapes 3, 4, 5: waves outer (8 x 4, 16 x 2, 4 x 8), dimension.receive
-// dimension.receive needs waves outer, dimension.transmit/none channels outer;
-// dimension.both runs with any of the first three.  A sub-tile of complex data whose windows
-// do not fit 80-entry slots runs half-size stages with 160-entry slots (half the
-// channels of a waves-outer stage, half the waves of a channels-outer one) in the same
-// buffers; real entries are half as large and always have 160-entry slots.
 template <int SHAPE>
-struct Shape;
-template <>
-struct Shape<0> {
-    static constexpr bool WAVES_OUTER = true;
-    static constexpr int CG = 2, KW = 16;
-};
-template <>
-struct Shape<1> {
-    static constexpr bool WAVES_OUTER = false;
-    static constexpr int CG = 8, KW = 4;
-};
-template <>
-struct Shape<2> {
-    static constexpr bool WAVES_OUTER = false;
-    static constexpr int CG = 16, KW = 2;
-};
-template <>
-struct Shape<3> {
-    static constexpr bool WAVES_OUTER = true;
-    static constexpr int CG = 8, KW = 4;
-};
-template <>
-struct Shape<4> {
-    static constexpr bool WAVES_OUTER = true;
-    static constexpr int CG = 16, KW = 2;
-};
-template <>
-struct Shape<5> {
-    static constexpr bool WAVES_OUTER = true;
-    static constexpr int CG = 4, KW = 8;
+struct Shape {
+    static constexpr bool WAVES_OUTER = kShapes[SHAPE].waves_outer;
+    static constexpr int CG = kShapes[SHAPE].cg, KW = kShapes[SHAPE].kw;
 };
 template <int SHAPE, bool BIG, bool WIDE>
 struct Stage {
@@ -342,38 +307,6 @@ struct Stage {
     static constexpr int SLOT = (WIDE || !BIG) ? 160 : 80;  // entries per (channel, wave) window
     static_assert(CG * KW * SLOT * (BIG ? 16 : 8) == kBufBytes, "a stage fills one buffer");
 };
-
-// Shared memory of one CTA: kRing stage buffers, then the per-tile tables (their size
-// depends on N, W and the stage shape).  1024 channels x 25 waves leave room for two
-// CTAs per SM.
-constexpr size_t kBuffers = (size_t)kRing * kBufBytes;
-
-// Byte offsets of the per-tile tables (16-byte records first).
-struct TileTables {
-    size_t el4, txc, txp, win_w, rxp, base_w, len_n, olist, kind_w, total;
-};
-
-// Per-channel tables hold NP and per-wave tables WP records, the counts rounded up to
-// whole stages: the channels / waves past N / W are padding with zero weight, so a
-// stage never needs bounds checks.
-template <int SHAPE>
-__host__ __device__ __forceinline__ TileTables tile_tables(int64_t NP, int64_t WP) {
-    // counts of channel groups and wave chunks, of the smaller stages where there are two
-    const int64_t NG = NP / Stage<SHAPE, true, true>::CG, NC = WP / Stage<SHAPE, true, true>::KW;
-    TileTables t;
-    size_t o = 0;
-    t.el4 = o;    o += 16 * NP;        // float4 per channel: x, y, z, delay base
-    t.txc = o;    o += 16 * WP;        // float4 per wave: delay coefficients
-    t.txp = o;    o += 16 * WP;        // float4 per wave: phase offset, apodization, fs/c, window offset
-    t.win_w = o;  o += 8 * WP;         // {window start, its largest position as a float (sign bit: inactive)} per wave
-    t.rxp = o;    o += 8 * NP;         // float2 per channel: phase (cycles) of the delay base, window offset
-    t.base_w = o; o += 4 * WP;         // delay base of each wave
-    t.len_n = o;  o += 4 * NP;         // largest window position of each channel (< 0: inactive)
-    t.olist = o;  o += 2 * (NG + NC);  // active outer indices, then active inner indices (16 bits)
-    t.kind_w = o; o += WP;
-    t.total = (o + 15) & ~size_t(15);
-    return t;
-}
 
 // Once per CTA: zero the stage buffers, so that units whose sums nothing takes (idle lanes,
 // inactive channels), which may read past a window's end, never read uninitialised words.
@@ -421,7 +354,7 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     Entry* slots = reinterpret_cast<Entry*>(smem);
     constexpr int CGM = Shape<SHAPE>::CG, KWM = Shape<SHAPE>::KW;
     const int NP = ((int)N + CGM - 1) / CGM * CGM, WP = ((int)W + KWM - 1) / KWM * KWM;
-    const TileTables tt = tile_tables<SHAPE>(NP, WP);
+    const TileTables tt = tile_tables(kShapes[SHAPE], NP, WP);
     unsigned char* tb = smem + kBuffers;
     float4* el4 = reinterpret_cast<float4*>(tb + tt.el4);
     float4* txc = reinterpret_cast<float4*>(tb + tt.txc);
@@ -464,8 +397,8 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
     const int32_t p_own = __ldg(tl + sub * kThreads + tid);
     const int32_t p_anchor = __ldg(tl);
     // this thread's pixel of the other sub-tile: the delay bases are the whole tile's
-    static_assert(kSub == 2, "one other sub-tile");
-    const int32_t p_other = __ldg(tl + (sub ^ 1) * kThreads + tid);
+    static_assert(kSub <= 2, "one other sub-tile");
+    const int32_t p_other = kSub == 2 ? __ldg(tl + (sub ^ 1) * kThreads + tid) : -1;
     const bool live = in_image(p_own), live_o = in_image(p_other);
     if (tid == 0) {
         s_tx_general = A.tx_apo_tab != nullptr || A.tx_delay_tab != nullptr;
@@ -1282,12 +1215,12 @@ __device__ __forceinline__ void das_tile(const Params& A, int tile, int sub, int
 
 // One launch per request: grid = (tiles x sub-tiles x CTAs per sub-tile, frames).
 template <int MODE, int ENT, bool EPI, int SHAPE>
-__global__ void __launch_bounds__(kThreads, 2) das_fast_kernel(const Params A) {
+__global__ void __launch_bounds__(kThreads, kSub) das_fast_kernel(const Params A) {
     const int b = (int)(blockIdx.x / A.split), part = A.split >= 2 ? (int)(blockIdx.x % A.split) : -1;
     das_tile<MODE, ENT, EPI, SHAPE>(A, b / kSub, b % kSub, (int64_t)blockIdx.y, part);
 }
 
-// Persistent form: two CTAs per SM pull (request, half tile, frames) work items from a
+// Persistent form: the CTAs that fit the SMs pull (request, half tile, frames) work items from a
 // queue counter until the batch is done, so requests of different scans, channel
 // counts and frame counts share one launch and balance across SMs.  An item is half a
 // tile over up to 8 consecutive frames of a request (fewer while that leaves each CTA
@@ -1301,7 +1234,7 @@ struct BatchParams {
 };
 
 template <int MODE, int ENT, bool EPI, int SHAPE>
-__global__ void __launch_bounds__(kThreads, 2) das_fast_persistent(const __grid_constant__ BatchParams B) {
+__global__ void __launch_bounds__(kThreads, kSub) das_fast_persistent(const __grid_constant__ BatchParams B) {
     __shared__ long long s_item;
     bool first = true;
     const int64_t total = B.first_item[B.n];
@@ -1321,12 +1254,6 @@ __global__ void __launch_bounds__(kThreads, 2) das_fast_persistent(const __grid_
         das_tile<MODE, ENT, EPI, SHAPE, true>(A, b / kSub, b % kSub, f0, -1, (int)min((int64_t)A.fpi, A.F - f0), first);
         first = false;
     }
-}
-
-template <int SHAPE>
-size_t smem_bytes(int64_t N, int64_t W) {
-    constexpr int CG = Shape<SHAPE>::CG, KW = Shape<SHAPE>::KW;
-    return kBuffers + tile_tables<SHAPE>((N + CG - 1) / CG * CG, (W + KW - 1) / KW * KW).total;
 }
 
 // Launch with leave to start while the kernel before it in the stream ends: the CTAs set
@@ -1349,7 +1276,7 @@ cudaError_t launch_dependent(K* kern, dim3 grid, size_t smem, cudaStream_t s, co
 
 template <int MODE, int ENT, bool EPI, int SHAPE>
 int launch(const Params& A, int64_t n_tiles, int64_t F, cudaStream_t s) {
-    const size_t smem = smem_bytes<SHAPE>(A.N, A.W);
+    const size_t smem = smem_bytes(SHAPE, A.N, A.W);
     auto kern = das_fast_kernel<MODE, ENT, EPI, SHAPE>;
     size_t limit = 0;
     const int rc = shared_limit((const void*)kern, limit);
@@ -1378,8 +1305,12 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t nct = (max_ctas > 0 ? std::min(max_ctas, sms) : sms) * (int64_t)kSub;
     size_t smem = 0;
+    for (int i = 0; i < n; ++i) smem = std::max(smem, smem_bytes(SHAPE, reqs[i].N, reqs[i].W));
+    int fit = 0;
+    int rc = ctas_per_sm(smem, fit);
+    if (rc) return rc;
+    const int64_t nct = (max_ctas > 0 ? std::min(max_ctas, sms) : sms) * (int64_t)std::min(fit, kSub);
     for (int i = 0; i < n; ++i) {
         B.req[i] = reqs[i];
         // frames per work item: up to kItemFrames, while every CTA keeps at least 8 items of the request
@@ -1387,17 +1318,16 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
         const int64_t fpi = std::max<int64_t>(1, std::min<int64_t>(kItemFrames, subs * frames[i] / (8 * nct)));
         B.req[i].fpi = (int)fpi;
         B.first_item[i + 1] = B.first_item[i] + subs * ((frames[i] + fpi - 1) / fpi);
-        smem = std::max(smem, smem_bytes<SHAPE>(reqs[i].N, reqs[i].W));
     }
     if (B.first_item[n] == 0) return USTB_OK;
     auto kern = das_fast_persistent<MODE, ENT, EPI, SHAPE>;
     size_t limit = 0;
-    const int rc = shared_limit((const void*)kern, limit);
+    rc = shared_limit((const void*)kern, limit);
     if (rc) return rc;
     USTB_REQUIRE(smem <= limit, USTB_E_SHAPE, "a request needs %zu bytes of shared memory per tile (limit %zu)", smem,
                  limit);
     USTB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s));
-    // two CTAs per SM, or fewer (max_ctas pairs) to leave room to launches on other streams
+    // as many CTAs as the SMs hold, or fewer (max_ctas SMs) to leave room to launches on other streams
     const unsigned grid = (unsigned)std::min<int64_t>(B.first_item[n], nct);
     kern<<<grid, kThreads, smem, s>>>(B);
     USTB_CUDA(cudaGetLastError());
@@ -1407,9 +1337,10 @@ int launch_batch(const Params* reqs, const int64_t* frames, int n, unsigned long
 }  // namespace
 
 // Kernel variant of (dimension, epilogue, stage shape) for one request kind.
-template <int ENT, bool BATCH>
+template <int ENT, bool BATCH, int SUBS>
 int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t* frames, int n,
              unsigned long long* counter, int64_t nt, int64_t F, cudaStream_t s, int max_ctas) {
+    static_assert(SUBS == kSub, "the including file sets the number");
     auto run = [&](auto m, auto e, auto sh) {
         constexpr int M = decltype(m)::value, S = decltype(sh)::value;
         constexpr bool E = decltype(e)::value;
