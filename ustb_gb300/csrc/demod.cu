@@ -14,7 +14,7 @@
 // sine and cosine per sample) with complex taps, at the same 2 FMA per tap and output.
 //
 // One CTA computes kout (<= 1024) consecutive outputs of tp traces (as many as fill its
-// threads) and loops over trace groups, so the complex taps are formed once per CTA.  It
+// threads, fewer where that leaves SMs without a CTA) and loops over trace groups, so the complex taps are formed once per CTA.  It
 // stages the samples that the outputs need in shared memory in polyphase order
 // (phase-major): output o reads, for tap k, position o + (last - k)/D of row (last - k) % D,
 // so the taps of one row step one position at a time.  Each thread forms two runs of 4
@@ -114,7 +114,7 @@ __device__ __forceinline__ void store_iq<__nv_bfloat16>(__nv_bfloat16* out, int6
 struct DemodArgs {
     int64_t L, Ld, n_traces, chunks, groups;  // chunks of kout outputs per trace, groups of (chunk, tp traces)
     int D, ntaps, kout;
-    int tp, tpt;           // traces per CTA, threads per trace
+    int tp, tpt, threads;  // traces per CTA, threads per trace and of a CTA
     int mb, shift;         // zero-phase: taps of the reference filter, and mb - 1
     int Qp, Cap;           // padded row stride (words); taps per polyphase row (a multiple of kTB)
     int raw;               // samples copied ahead per trace (a multiple of 4)
@@ -411,8 +411,11 @@ __global__ void __launch_bounds__(kThreads, 4) demod_kernel(const S* __restrict_
 
 // The split of the work: outputs per trace and CTA (the trace's Ld outputs in the fewest
 // equal chunks: a last, short chunk would leave most of its CTA idle), threads per trace
-// and as many traces as fill the CTA's threads and its shared memory.
-void plan_demod(DemodArgs& a, bool zp, bool vec) {
+// and as many traces as fill the CTA's threads and its shared memory, or few enough that
+// every SM has a group (128 traces of 645 samples, in a graph: 31 taps, decimation 2, 5.8 us
+// with full CTAs, 4.8; zero phase 11.9, 8.5; 256 of 1536, zero phase, 10.0, 9.6; with 64
+// threads to such a CTA 4.9, 10.6 and 10.0).
+void plan_demod(DemodArgs& a, bool zp, bool vec, int sms) {
     const int64_t kmax = std::max<int64_t>(32, std::min<int64_t>(kOutMax, (kStage - a.ntaps) / a.D));
     a.chunks = (a.Ld + kmax - 1) / kmax;
     a.kout = (int)((a.Ld + a.chunks - 1) / a.chunks);
@@ -425,20 +428,23 @@ void plan_demod(DemodArgs& a, bool zp, bool vec) {
     a.edges = zp ? std::max(1, (a.mb - 2) / a.D + 1) : 0;
     a.vec = vec ? 1 : 0;
     const int64_t per_trace = (int64_t)a.D * a.Qp + a.raw + 2 * a.kout + (zp ? 4 * (a.mb - 1) + 4 * a.edges : 0);
-    a.tp = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)kThreads / a.tpt, 12288 / per_trace, a.n_traces}));
+    const int64_t fill = std::max<int64_t>(1, std::min<int64_t>((int64_t)kThreads / a.tpt, 12288 / per_trace));
+    const int64_t each = (a.n_traces * a.chunks + sms - 1) / sms;  // a group for every SM
+    a.tp = (int)std::min(fill, each);
+    // a CTA of fewer traces keeps the threads: they form its taps and leave its outputs
+    a.threads = each < fill ? kThreads : (a.tp * a.tpt + 31) / 32 * 32;
     a.groups = (a.n_traces + a.tp - 1) / a.tp * a.chunks;
 }
 
 
 template <typename S, bool ZP>
 int launch_demod(const S* rf, void* iq, int32_t dst_type, const float* taps, DemodArgs a, cudaStream_t s) {
-    plan_demod(a, ZP, ((uintptr_t)rf & (4 * sizeof(S) - 1)) == 0);
-    USTB_REQUIRE(a.groups <= INT32_MAX, USTB_E_SHAPE, "too many traces x output chunks");
-    const size_t smem = sizeof(float) * demod_layout(a, ZP).total;
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const unsigned threads = (unsigned)((a.tp * a.tpt + 31) / 32 * 32);
+    plan_demod(a, ZP, ((uintptr_t)rf & (4 * sizeof(S) - 1)) == 0, sms);
+    USTB_REQUIRE(a.groups <= INT32_MAX, USTB_E_SHAPE, "too many traces x output chunks");
+    const size_t smem = sizeof(float) * demod_layout(a, ZP).total;
     const unsigned blocks = (unsigned)std::min<int64_t>(a.groups, (int64_t)sms * 16);
     auto start = [&](auto kern, auto* dst) -> int {
         size_t limit = 0;
@@ -446,7 +452,7 @@ int launch_demod(const S* rf, void* iq, int32_t dst_type, const float* taps, Dem
         if (rc) return rc;
         USTB_REQUIRE(smem <= limit, USTB_E_SHAPE, "decimation %d with %d taps needs %zu bytes of shared memory", a.D,
                      a.ntaps, smem);
-        kern<<<blocks, threads, smem, s>>>(rf, dst, taps, a);
+        kern<<<blocks, a.threads, smem, s>>>(rf, dst, taps, a);
         USTB_CUDA(cudaGetLastError());
         return USTB_OK;
     };
