@@ -617,9 +617,12 @@ __global__ void __launch_bounds__(kThreads) das_table_few_waves(const TableArgs 
 //   160,000 pixels 128 x 75: complex both 1199 / 1079
 //   40,000 pixels 64 x 16 x 2 frames (2 per SM): complex receive 70 / 75
 //   320,000 pixels 64 x 16: complex both 283 / 314, receive 306 / 442
-// Complex both of up to 12 waves stays in one part where all its CTAs are resident in one
-// full round (2 to 4 per SM): 41,184 pixels of a volume, 529 channels x 4 waves, 598 / 631;
-// 45,450 pixels 41 x 10 x 2 frames 137 / 144; 74,572 pixels 58 x 4 67 / 70.
+// Complex both of one frame and one chunk of waves stays in one part where its CTAs nearly
+// fill one round (four are resident on an SM; with more frames three, so a second round
+// follows): 75,878 pixels (3.9 per SM) 128 x 4 57 / 62, 128 x 8 61 / 66, 40 x 4 39 / 43, but
+// 128 x 12 107 / 102, 128 x 8 x 2 frames 172 / 138; 60,314 pixels (3.1) 128 x 4 58 / 49;
+// 40,858 (2.1) 52 / 36, 128 x 12 99 / 60; a volume's 57,200 pixels, 529 channels x 4 waves,
+// 480 / 458.
 // A part needs channels of its own (chunks of WC).
 int in_parts(int mode, bool cplx, const TableArgs& A, bool& parts) {
     int dev = 0, sms = 0;
@@ -630,7 +633,7 @@ int in_parts(int mode, bool cplx, const TableArgs& A, bool& parts) {
                            : (mode == USTB_DIM_BOTH && cplx) || (mode == USTB_DIM_TRANSMIT && !few) ? 9
                                                                                                         : 5;
     const int64_t ctas = (A.P + kThreads - 1) / kThreads;
-    const bool one_round = mode == USTB_DIM_BOTH && cplx && !few && A.W <= 12 && ctas > 2 * sms && ctas <= 4 * sms;
+    const bool one_round = mode == USTB_DIM_BOTH && cplx && !few && A.F == 1 && A.W <= WC && 2 * ctas > 7 * sms && ctas <= 4 * sms;
     parts = A.N >= 4 * WC && ctas <= per_sm * sms && !one_round;
     return USTB_OK;
 }
