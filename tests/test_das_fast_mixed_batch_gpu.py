@@ -56,6 +56,14 @@ def test_stages_asked_for_stay(cuda_dev):
     assert launches(fast.das_fast_batch(reqs)) == 2
 
 
+def test_library_stages_asked_for_share(cuda_dev):
+    """The shape that the library would choose, asked for (as tuned plans do)."""
+    rng = np.random.default_rng(10)
+    reqs = [request(rng, p, 5, True, 3, False, cuda_dev, shape=s)
+            for p, s in ((Precision.fp16, 0), (Precision.fp32, 2), (Precision.bf16, 2))]
+    assert launches(fast.das_fast_batch(reqs)) == 1
+
+
 def test_many_items_keep_their_variants(cuda_dev):
     rng = np.random.default_rng(9)
     reqs = [request(rng, p, 1 + i % 2 * 3, True, 1, False, cuda_dev, F=600) for i in range(2) for p in (Precision.fp32,)]

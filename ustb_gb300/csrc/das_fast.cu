@@ -530,7 +530,7 @@ static int share_variants(const ustb_das_request* reqs, int32_t n, const std::ve
                 auto member = [&](int i) {
                     const ustb_das_request& q = reqs[i];
                     return key[i] >= 0 && q.dimension == dim && (q.epilogue != 0) == (epi != 0) && q.is_complex == cplx &&
-                           q.geometry->stage_shape == 0;
+                           P[i].shape == shape_for(dim, cplx != 0, 0, q.W);  // the library's, or the same asked for
                 };
                 int first = -1;
                 bool differ = false;
