@@ -170,7 +170,7 @@ enum {
     USTB_WIN_TUKEY25 = 4, USTB_WIN_TUKEY50 = 5, USTB_WIN_TUKEY75 = 6, USTB_WIN_TRIANGLE = 9
 };
 
-/* Pixels per tile of the fast path (two CTAs). */
+/* Pixels per tile of the fast path (two CTAs, or one). */
 #define USTB_TILE_PIXELS 512
 
 /*

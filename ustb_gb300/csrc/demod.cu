@@ -27,7 +27,7 @@
 // length.  The outputs leave through shared memory, so that the stores are contiguous.
 //
 // Instruction-bound (75 % issue; HBM would take 51 us).  GB300, a call on 56320 int16 traces
-// of 1536 samples, 30 taps, decimation 2, half-precision output: 284 us (515 us with a
+// of 1536 samples, 31 taps, decimation 2, half-precision output: 284 us (515 us with a
 // mixed complex sample staged per input sample); zero phase, 14080 float traces of 1536,
 // 129 taps, decimation 4: 164 us (246 us).
 //
