@@ -210,7 +210,8 @@ typedef struct {
     int32_t stage_shape;         /* (channel, wave) pairs per shared-memory stage and loop order:
                                     1 = waves outer, 2 channels x 16 waves (dimension.both / receive);
                                     2 = channels outer, 8 x 4; 3 = channels outer, 16 x 2
-                                    (dimension.both / transmit / none); 0 = the library's choice */
+                                    (dimension.both / transmit / none); 0 = the library's choice,
+                                    which persistent launches of complex data always take */
 } ustb_das_geometry;
 
 /* Outputs of ustb_das_fast (device pointers; unused ones NULL). */
@@ -286,7 +287,7 @@ typedef struct {
  * (frame, tile) work items and the CTAs that fit the SMs pull items from a queue until all
  * are done, so requests of different scans, probes, frame counts and sizes share
  * one launch and balance across the GPU (one launch per dimension / real-complex /
- * epilogue combination and stage_shape present; batches of more than 16 work items per
+ * epilogue combination, and stage_shape of real data, present; batches of more than 16 work items per
  * persistent CTA also launch once per kind of entries and of receive stages, which differ
  * with the storage type and the number of waves).  Each request's
  * entry array (see ustb_das_fast) lives in library scratch until the launches are done.  The

@@ -49,11 +49,17 @@ def test_few_items_share_a_launch(cuda_dev, dim, cplx, epi, workspace):
             assert torch.linalg.vector_norm((y - alone[k])[ok]) <= 1e-6 * torch.linalg.vector_norm(alone[k][ok]), k
 
 
-def test_stages_asked_for_stay(cuda_dev):
-    """A request with a stage shape of its own keeps it, in a launch of its own."""
+@pytest.mark.parametrize("cplx, dim, expect", [(False, 1, 2), (True, 1, 1), (True, 3, 1), (True, 2, 1)])
+def test_stages_asked_for(cuda_dev, cplx, dim, expect):
+    """A request of real data with a stage shape of its own keeps it, in a launch of its own;
+    complex data takes the library's."""
     rng = np.random.default_rng(9)
-    reqs = [request(rng, Precision.fp32, W, True, 1, False, cuda_dev, shape=s) for W, s in ((1, 0), (20, 0), (5, 1))]
-    assert launches(fast.das_fast_batch(reqs)) == 2
+    reqs = [request(rng, Precision.fp32, W, cplx, dim, False, cuda_dev, shape=s)
+            for W, s in ((1, 0), (20, 0), (5, 1 if dim == 1 else 3))]
+    assert launches(fast.das_fast_batch(reqs)) == expect
+    for r in reqs:
+        alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, dim, L=L)["cube"]
+        assert torch.linalg.vector_norm(r.outputs["cube"] - alone) <= 1e-6 * torch.linalg.vector_norm(alone)
 
 
 def test_library_stages_asked_for_share(cuda_dev):

@@ -567,7 +567,11 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
     uint32_t* flags = reinterpret_cast<uint32_t*>(scratch);
     USTB_CUDA(cudaMemsetAsync(scratch, 0, sizeof(uint64_t), s));
     if (n == 0) return USTB_OK;
-    // validate all requests first, then launch one persistent kernel per kernel variant
+    // validate all requests first, then launch one persistent kernel per kernel variant.
+    // Complex data takes the library's stages: beside the loop over frames the sums of the
+    // others spill (2 x 16: 1.7 KB a thread, 16 x 2 1.2 KB).  128 channels on 256 x 256 pixels,
+    // 2 x 16 / 16 x 2 / 8 x 4, us: 5 waves 80 / 79 / 64, 16 waves 115 / 134 / 110, 75 waves
+    // 495 / 469 / 399.
     std::vector<Params> P(n);
     std::vector<int64_t> frames(n);
     std::vector<int> key(n, -1);
@@ -583,7 +587,14 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
             return rc;
         }
         frames[i] = q.F;
-        if (!empty) key[i] = 0;
+        if (empty) continue;
+        key[i] = 0;
+        if (q.is_complex) {  // the library's own stages
+            P[i].shape = shape_for(q.dimension, true, 0, q.W);
+            P[i].ent = entries_for(q.storage, true, q.dimension, P[i].shape, q.W);
+            rc = subs_for(P[i], q.dimension);
+            if (rc) return rc;
+        }
     }
     int rc = share_variants(reqs, n, key, P);
     if (rc) return rc;

@@ -1349,38 +1349,41 @@ int das_dispatch(int dim, int epi, int shape, const Params* reqs, const int64_t*
     };
 #define USTB_RUN(M, E, S) \
     return run(std::integral_constant<int, M>{}, std::integral_constant<bool, E>{}, std::integral_constant<int, S>{})
-    if constexpr (ENT == kEntHalf || ENT == kEntBf16) {  // only the library's own shapes (entries_for)
-        switch (dim) {
-            case USTB_DIM_RECEIVE: USTB_RUN(USTB_DIM_RECEIVE, false, 3);
-            case USTB_DIM_TRANSMIT:
-                if (epi) USTB_RUN(USTB_DIM_TRANSMIT, true, 1);
-                USTB_RUN(USTB_DIM_TRANSMIT, false, 1);
-            default: USTB_RUN(USTB_DIM_BOTH, false, 1);
+    constexpr bool k16 = ENT == kEntHalf || ENT == kEntBf16;        // (entries_for: the library's shapes only)
+    constexpr bool kOwn = k16 || (BATCH && ENT == kEntComplex);     // (as das_fast_batch_impl sets them)
+    if constexpr (SUBS == 2) {  // (subs_for: whole tiles for dimension.both only)
+        if constexpr (!k16)
+            if (dim == USTB_DIM_NONE) {
+                if constexpr (!kOwn)
+                    if (shape == 2) USTB_RUN(USTB_DIM_NONE, false, 2);
+                USTB_RUN(USTB_DIM_NONE, false, 1);
+            }
+        if (dim == USTB_DIM_RECEIVE) {
+            if constexpr (!k16) {
+                if (shape == 4) USTB_RUN(USTB_DIM_RECEIVE, false, 4);
+                if (shape == 5) USTB_RUN(USTB_DIM_RECEIVE, false, 5);
+            }
+            if constexpr (!kOwn)
+                if (shape == 0) USTB_RUN(USTB_DIM_RECEIVE, false, 0);
+            USTB_RUN(USTB_DIM_RECEIVE, false, 3);
         }
-    } else {
-    switch (dim) {
-        case USTB_DIM_NONE:
-            if (shape == 2) USTB_RUN(USTB_DIM_NONE, false, 2);
-            USTB_RUN(USTB_DIM_NONE, false, 1);
-        case USTB_DIM_RECEIVE:
-            if (shape == 3) USTB_RUN(USTB_DIM_RECEIVE, false, 3);
-            if (shape == 4) USTB_RUN(USTB_DIM_RECEIVE, false, 4);
-            if (shape == 5) USTB_RUN(USTB_DIM_RECEIVE, false, 5);
-            USTB_RUN(USTB_DIM_RECEIVE, false, 0);
-        case USTB_DIM_TRANSMIT:
-            if constexpr (ENT == kEntComplex)
+        if (dim == USTB_DIM_TRANSMIT) {
+            if constexpr (ENT != kEntReal)
                 if (epi) {
-                    if (shape == 2) USTB_RUN(USTB_DIM_TRANSMIT, true, 2);
+                    if constexpr (!kOwn)
+                        if (shape == 2) USTB_RUN(USTB_DIM_TRANSMIT, true, 2);
                     USTB_RUN(USTB_DIM_TRANSMIT, true, 1);
                 }
-            if (shape == 2) USTB_RUN(USTB_DIM_TRANSMIT, false, 2);
+            if constexpr (!kOwn)
+                if (shape == 2) USTB_RUN(USTB_DIM_TRANSMIT, false, 2);
             USTB_RUN(USTB_DIM_TRANSMIT, false, 1);
-        default:
-            if (shape == 0) USTB_RUN(USTB_DIM_BOTH, false, 0);
-            if (shape == 2) USTB_RUN(USTB_DIM_BOTH, false, 2);
-            USTB_RUN(USTB_DIM_BOTH, false, 1);
+        }
     }
+    if constexpr (!kOwn) {
+        if (shape == 0) USTB_RUN(USTB_DIM_BOTH, false, 0);
+        if (shape == 2) USTB_RUN(USTB_DIM_BOTH, false, 2);
     }
+    USTB_RUN(USTB_DIM_BOTH, false, 1);
 #undef USTB_RUN
 }
 
