@@ -49,13 +49,13 @@ def test_few_items_share_a_launch(cuda_dev, dim, cplx, epi, workspace):
             assert torch.linalg.vector_norm((y - alone[k])[ok]) <= 1e-6 * torch.linalg.vector_norm(alone[k][ok]), k
 
 
-@pytest.mark.parametrize("cplx, dim, expect", [(False, 1, 2), (True, 1, 1), (True, 3, 1), (True, 2, 1)])
-def test_stages_asked_for(cuda_dev, cplx, dim, expect):
+@pytest.mark.parametrize("cplx, dim, asked, expect", [(False, 3, 1, 2), (True, 1, 1, 1), (True, 3, 3, 1), (True, 2, 3, 1)])
+def test_stages_asked_for(cuda_dev, cplx, dim, asked, expect):
     """A request of real data with a stage shape of its own keeps it, in a launch of its own;
     complex data takes the library's."""
     rng = np.random.default_rng(9)
     reqs = [request(rng, Precision.fp32, W, cplx, dim, False, cuda_dev, shape=s)
-            for W, s in ((1, 0), (20, 0), (5, 1 if dim == 1 else 3))]
+            for W, s in ((1, 0), (20, 0), (5, asked))]
     assert launches(fast.das_fast_batch(reqs)) == expect
     for r in reqs:
         alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, dim, L=L)["cube"]
@@ -74,3 +74,18 @@ def test_many_items_keep_their_variants(cuda_dev):
     rng = np.random.default_rng(9)
     reqs = [request(rng, p, 1 + i % 2 * 3, True, 1, False, cuda_dev, F=600) for i in range(2) for p in (Precision.fp32,)]
     assert launches(fast.das_fast_batch(reqs)) == 2
+
+
+@pytest.mark.parametrize("cplx", [True, False])
+@pytest.mark.parametrize("W, F", [(1, 1), (9, 1), (20, 2), (75, 3), (3, 400)])
+def test_one_receive_image(cuda_dev, W, F, cplx):
+    """Less than a round of work items: a grid launch (no queue counter), the same result;
+    with a bound on the CTAs, and with many frames, the persistent one."""
+    rng = np.random.default_rng(W)
+    r = request(rng, Precision.fp32, W, cplx, 1, False, cuda_dev, F=F)
+    alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, 1, F=F, L=L)["cube"]
+    for max_ctas, expect in ((0, int(F == 400)), (3, 1)):
+        ws = torch.empty(fast.workspace_bytes([r]), dtype=torch.uint8, device=cuda_dev)
+        scratch = fast.das_fast_batch([r], workspace=ws, max_ctas=max_ctas)
+        assert launches(scratch) == expect and int(scratch[0]) == 0
+        assert torch.linalg.vector_norm(r.outputs["cube"] - alone) <= 1e-6 * torch.linalg.vector_norm(alone)
