@@ -287,14 +287,15 @@ typedef struct {
  * (frame, tile) work items and the CTAs that fit the SMs pull items from a queue until all
  * are done, so requests of different scans, probes, frame counts and sizes share
  * one launch and balance across the GPU (one launch per dimension / real-complex /
- * epilogue combination, and stage_shape of real data, present; batches of more than 16 work items per
- * persistent CTA also launch once per kind of entries and of receive stages, which differ
- * with the storage type and the number of waves).  Each request's
+ * epilogue combination, and stage_shape of real data, present; batches of more than 16
+ * work items per persistent CTA also launch once per kind of entries and of receive
+ * stages, which differ with the storage type and the number of waves).  Each request's
  * entry array (see ustb_das_fast) lives in library scratch until the launches are done.  The
  * reference runs requests one at a time (+midprocess/das.m:77-317,
  * +mex/source/das_cuda.cu:253-283 pipelines only frames).
  * scratch: device memory of at least 8*(n+1) bytes; word 0 receives the
  * USTB_FLAG_* bits of all requests (low 32 bits), words 1.. are queue counters.
+ * Few work items may run as ustb_das_fast's grid launches instead (no counter is used).
  * Stream-ordered; results are as ustb_das_fast gives them for each request.
  */
 int ustb_das_fast_batch(const ustb_das_request* reqs, int32_t n, uint64_t* scratch, void* stream);

@@ -61,7 +61,7 @@ def test_parts_asked_for(cuda_dev, parts):
 def test_one_launch_beside_few_channels(cuda_dev):
     made = [case(n, n, 3, 1, True, Precision.fp16, cuda_dev) for n in (35, 9)]
     reqs = [fast.Request(st, Precision.fp16, True, g, 3, L=L - 2) for g, st, _ in made]
-    scratch = fast.das_fast_batch(reqs)
+    scratch = fast.das_fast_batch(reqs, max_ctas=9)  # (bounded: persistent)
     assert int((scratch[1:] != 0).sum()) == 1
     for r, (_, _, want) in zip(reqs, made):
         w = want(3)

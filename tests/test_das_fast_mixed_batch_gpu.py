@@ -56,7 +56,7 @@ def test_stages_asked_for(cuda_dev, cplx, dim, asked, expect):
     rng = np.random.default_rng(9)
     reqs = [request(rng, Precision.fp32, W, cplx, dim, False, cuda_dev, shape=s)
             for W, s in ((1, 0), (20, 0), (5, asked))]
-    assert launches(fast.das_fast_batch(reqs)) == expect
+    assert launches(fast.das_fast_batch(reqs, max_ctas=4)) == expect  # (bounded: persistent)
     for r in reqs:
         alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, dim, L=L)["cube"]
         assert torch.linalg.vector_norm(r.outputs["cube"] - alone) <= 1e-6 * torch.linalg.vector_norm(alone)
@@ -76,16 +76,30 @@ def test_many_items_keep_their_variants(cuda_dev):
     assert launches(fast.das_fast_batch(reqs)) == 2
 
 
-@pytest.mark.parametrize("cplx", [True, False])
-@pytest.mark.parametrize("W, F", [(1, 1), (9, 1), (20, 2), (75, 3), (3, 400)])
-def test_one_receive_image(cuda_dev, W, F, cplx):
-    """Less than a round of work items: a grid launch (no queue counter), the same result;
-    with a bound on the CTAs, and with many frames, the persistent one."""
+@pytest.mark.parametrize("dim, cplx, epi", [(3, True, False), (3, False, False), (2, True, False), (2, False, False),
+                                            (2, True, True), (1, True, False), (1, False, False)])
+@pytest.mark.parametrize("precision", [Precision.fp32, Precision.fp16])
+@pytest.mark.parametrize("W, F", [(1, 1), (20, 2), (75, 3), (3, 400)])
+def test_one_small_request(cuda_dev, W, F, precision, dim, cplx, epi):
+    """Fewer work items than SMs: a grid launch in parts where that is faster, with scratch
+    from the pool or from what a workspace has left; with a bound on the CTAs, and with many
+    frames, the persistent one.  The same result every way, and every time."""
     rng = np.random.default_rng(W)
-    r = request(rng, Precision.fp32, W, cplx, 1, False, cuda_dev, F=F)
-    alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, 1, F=F, L=L)["cube"]
-    for max_ctas, expect in ((0, int(F == 400)), (3, 1)):
-        ws = torch.empty(fast.workspace_bytes([r]), dtype=torch.uint8, device=cuda_dev)
-        scratch = fast.das_fast_batch([r], workspace=ws, max_ctas=max_ctas)
-        assert launches(scratch) == expect and int(scratch[0]) == 0
-        assert torch.linalg.vector_norm(r.outputs["cube"] - alone) <= 1e-6 * torch.linalg.vector_norm(alone)
+    r = request(rng, precision, W, cplx, dim, epi, cuda_dev, F=F)
+    alone = fast.das_fast(r.ch, r.precision, cplx, r.geom, dim, F=F, L=L, epilogue=epi)
+    bytes_ = fast.workspace_bytes([r])
+    for extra, max_ctas in ((None, 0), (0, 0), (1 << 22, 0), (0, 3)):
+        ws = None if extra is None else torch.empty(bytes_ + extra, dtype=torch.uint8, device=cuda_dev)
+        counts = []
+        for _ in range(2):
+            scratch = fast.das_fast_batch([r], workspace=ws, max_ctas=max_ctas)
+            assert int(scratch[0]) == 0
+            counts.append(launches(scratch))
+        assert counts[0] == counts[1] and (counts[0] == 1 or (max_ctas == 0 and F < 400))
+        if W == 75 and extra != 0:
+            assert counts[0] == 0  # a grid launch has no queue counter
+        for k, y in r.outputs.items():
+            ok = torch.isfinite(alone[k].abs())
+            assert torch.equal(ok, torch.isfinite(y.abs()))
+            bar = 1e-6 if k == "cube" else 1e-5  # the factors square and divide sums of another order
+            assert torch.linalg.vector_norm((y - alone[k])[ok]) <= bar * torch.linalg.vector_norm(alone[k][ok]), k

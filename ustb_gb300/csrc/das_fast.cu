@@ -63,6 +63,17 @@ int shape_for(int dim, bool cplx, int32_t requested, int64_t W) {
     }
 }
 
+// A sub-tile's work in stages, and a CTA's that has one of `parts` of it.
+struct Work {
+    int64_t groups, chunks;
+    double setup;
+    double cta(int parts) const { return setup + (double)groups * (double)chunks / parts; }
+};
+Work work_of(const Params& A) {
+    const ustb::StageShape sh = ustb::kShapes[A.shape];
+    return {(A.N + sh.cg - 1) / sh.cg, (A.W + sh.kw - 1) / sh.kw, 4.5 + (double)(A.N + A.W) / 128.0};
+}
+
 // CTAs (parts) per sub-tile of a grid launch.  Few sub-tiles leave SMs without work or a
 // last round of long CTAs; each part sets the tile up again.  The number taken minimises
 //   (rounds + uneven) (set-up + stages / parts),
@@ -87,16 +98,13 @@ int parts_for(const Params& A, int dim, int32_t requested, int& parts) {
     int dev = 0, sms = 0;
     USTB_CUDA(cudaGetDevice(&dev));
     USTB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const ustb::StageShape sh = ustb::kShapes[A.shape];
-    const int64_t groups = (A.N + sh.cg - 1) / sh.cg, chunks = (A.W + sh.kw - 1) / sh.kw;
-    const int64_t most = dim == USTB_DIM_RECEIVE ? chunks : dim == USTB_DIM_TRANSMIT ? groups : groups * chunks / 4;
-    const double stages = (double)groups * (double)chunks;
-    const double setup = 4.5 + (double)(A.N + A.W) / 128.0;  // of a CTA, in stages
+    const Work w = work_of(A);
+    const int64_t most = dim == USTB_DIM_RECEIVE ? w.chunks : dim == USTB_DIM_TRANSMIT ? w.groups : w.groups * w.chunks / 4;
     const double rounds = (double)A.n_tiles * (double)A.F / sms;  // of one part each (A.subs CTAs per SM)
     double best = 0.0;
     for (int k = 1; k <= 8 && k <= most; ++k) {
         const double r = std::max(k * rounds, 1.0 / A.subs), uneven = 0.25 + 0.5 * std::min(std::max(1.5 - r, 0.0), 0.5);
-        const double cost = (r + uneven) * (setup + stages / k);
+        const double cost = (r + uneven) * w.cta(k);
         if (k == 1 || cost < 0.99 * best) {
             parts = k;
             best = cost;
@@ -557,6 +565,39 @@ static int share_variants(const ustb_das_request* reqs, int32_t n, const std::ve
     return USTB_OK;
 }
 
+// Scratch of a request's parts on a 256-byte boundary.
+static int64_t parts_room(int64_t sums, int64_t tickets) {
+    return (sums + tickets * (int64_t)sizeof(unsigned) + 255) & ~int64_t(255);
+}
+
+// Whether the requests of one variant run faster one after the other as grid launches, whose
+// parts fill the SMs, than as one persistent launch of whole sub-tiles.  With fewer of these
+// than SMs, the persistent launch takes as long as the longest request's one CTA, the grid
+// launches the sum of their parts' (and a launch each, about 3 stages).  `room`: bytes of a
+// caller's workspace left for the sums of parts, < 0: from the pool.  Persistent / grid, us:
+// receive images of 64 channels x 75 waves, 100 x 100 pixels x 3 frames, 535 / 272, x 16 waves
+// 122 / 63; 128 channels x 3 waves on 256 x 256 49 / 37; both, 64 x 75 on 50 x 50 328 / 90, 128 x
+// 16 on 256 x 256 111 / 80; transmit with factors, 64 x 16 on 50 x 50 101 / 42.
+static int grids_faster(const ustb_das_request& q, std::vector<Params>& gp, int sms, int64_t room, bool& yes) {
+    yes = false;
+    int64_t items = 0, need = 0;
+    double one = 0.0, all = 0.0;
+    for (Params& A : gp) {
+        items += A.n_tiles * A.F;
+        if (items > sms || q.dimension == USTB_DIM_NONE) return USTB_OK;
+        const int rc = parts_for(A, q.dimension, 0, A.split);
+        if (rc) return rc;
+        int64_t tickets = 0;
+        const int64_t sums = part_bytes(A, q.dimension, q.epilogue != 0, tickets);
+        need += parts_room(sums, tickets);
+        const Work w = work_of(A);
+        one = std::max(one, w.cta(1));
+        all += 3.0 + w.cta(A.split);
+    }
+    yes = all < 0.9 * one && (room < 0 || need <= room);
+    return USTB_OK;
+}
+
 static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t* scratch, void* workspace,
                                int64_t workspace_bytes, int32_t max_ctas, void* stream) {
     ustb::clear_error();
@@ -593,7 +634,6 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
             P[i].shape = shape_for(q.dimension, true, 0, q.W);
             P[i].ent = entries_for(q.storage, true, q.dimension, P[i].shape, q.W);
             rc = subs_for(P[i], q.dimension);
-            if (!rc) rc = parts_for(P[i], q.dimension, 0, P[i].split);
             if (rc) return rc;
         }
     }
@@ -650,19 +690,38 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
                 done[j] = true;
             }
         const ustb_das_request& q = reqs[i];
-        // One receive image of less than a round of work items: a grid launch, whose parts
-        // (disjoint outputs, no scratch) fill the SMs.  64 channels x 75 waves on 100 x 100
-        // pixels x 3 frames 535 us here, 272 there, x 16 waves 122 and 63; 128 channels x 3
-        // waves on 256 x 256 49 and 37.
-        if (gp.size() == 1 && q.dimension == USTB_DIM_RECEIVE && max_ctas == 0 &&
-            gp[0].n_tiles * gp[0].F <= sms) {
-            const int rc = dispatch<false>(q.dimension, 0, gp.data(), nullptr, 1, nullptr, gp[0].n_tiles, gp[0].F, s, 0);
-            if (rc) {
-                release();
-                return rc;
+        bool grids = false;
+        int rc = max_ctas > 0 ? (int)USTB_OK : grids_faster(q, gp, sms, workspace ? workspace_bytes - ws_off : -1, grids);
+        for (size_t k = 0; grids && !rc && k < gp.size(); ++k) {
+            Params& A = gp[k];
+            int64_t tickets = 0;
+            const int64_t sums = part_bytes(A, q.dimension, q.epilogue != 0, tickets);
+            const int64_t room = parts_room(sums, tickets);
+            void* scr = workspace ? static_cast<char*>(workspace) + ws_off : nullptr;
+            if (workspace) {
+                ws_off += room;
+            } else if (tickets) {
+                rc = pool_alloc(room, "partial sums", &scr, s);
+                if (!rc) ents.push_back(scr);
             }
-            continue;
+            if (rc == USTB_E_OOM) {  // whole sub-tiles
+                ustb::clear_error();
+                A.split = 1;
+                tickets = 0;
+                rc = USTB_OK;
+            }
+            if (tickets) {
+                set_parts(A, scr, sums);
+                const cudaError_t e = cudaMemsetAsync(A.tickets, 0, (size_t)tickets * sizeof(unsigned), s);
+                if (e != cudaSuccess) rc = ustb::cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
+            }
+            if (!rc) rc = dispatch<false>(q.dimension, q.epilogue, &A, nullptr, 1, nullptr, A.n_tiles, A.F, s, 0);
         }
+        if (rc) {
+            release();
+            return rc;
+        }
+        if (grids) continue;
         for (size_t off = 0; off < gp.size(); off += kMaxBatch) {
             const int cnt = (int)std::min<size_t>(kMaxBatch, gp.size() - off);
             unsigned long long* counter = reinterpret_cast<unsigned long long*>(scratch + 1 + group);
@@ -672,7 +731,7 @@ static int das_fast_batch_impl(const ustb_das_request* reqs, int32_t n, uint64_t
                 ustb::set_error("scratch holds n + 1 words");
                 return USTB_E_ARG;
             }
-            const int rc = dispatch<true>(q.dimension, q.epilogue, gp.data() + off, gf.data() + off, cnt, counter, 0, 0, s, max_ctas);
+            rc = dispatch<true>(q.dimension, q.epilogue, gp.data() + off, gf.data() + off, cnt, counter, 0, 0, s, max_ctas);
             if (rc) {
                 release();
                 return rc;
